@@ -564,10 +564,8 @@ __device__ __forceinline__ EdgeRange edge_range(const Args& A, int64_t i) {
 // Level-0 norms of one block of kNodeThreads threads (every thread arrives):
 // sums through shared memory, halving the active threads each step down to
 // one warp, so every FP64 add is a useful one (a shuffle tree in each warp
-// would issue five per thread); then one atomic per sum.  A NaN or infinity
-// stops the solver (euler3d.cpp:539-548).
-__device__ __forceinline__ void block_norms(double* srms, double* srho, int* sbad, double r2, double rr, int bad,
-                                            DevStatus* st) {
+// would issue five per thread).  Thread 0 returns true with the block's sums.
+__device__ __forceinline__ bool block_sums(double* srms, double* srho, int* sbad, double& r2, double& rr, int& bad) {
   const int t = threadIdx.x;
   srms[t] = r2;
   srho[t] = rr;
@@ -578,15 +576,21 @@ __device__ __forceinline__ void block_norms(double* srms, double* srho, int* sba
     if (t < w) { srms[t] += srms[t + w]; srho[t] += srho[t + w]; sbad[t] += sbad[t + w]; }
     __syncthreads();
   }
-  if (t < 32) {
-    r2 = warp_sum(srms[t]);
-    rr = warp_sum(srho[t]);
-    bad = warp_sum_int(sbad[t]);
-    if (t == 0) {
-      atomicAdd(&st->rms_acc, r2);
-      atomicAdd(&st->rho_acc, rr);
-      if (bad) { atomicAdd(&st->bad_count, bad); atomicOr(&st->halt, 1); }
-    }
+  if (t >= 32) return false;
+  r2 = warp_sum(srms[t]);
+  rr = warp_sum(srho[t]);
+  bad = warp_sum_int(sbad[t]);
+  return t == 0;
+}
+
+// ... added to a plain solver's norms with one atomic per sum.  A NaN or
+// infinity stops the solver (euler3d.cpp:539-548).
+__device__ __forceinline__ void block_norms(double* srms, double* srho, int* sbad, double r2, double rr, int bad,
+                                            DevStatus* st) {
+  if (block_sums(srms, srho, sbad, r2, rr, bad)) {
+    atomicAdd(&st->rms_acc, r2);
+    atomicAdd(&st->rho_acc, rr);
+    if (bad) { atomicAdd(&st->bad_count, bad); atomicOr(&st->halt, 1); }
   }
 }
 
@@ -646,9 +650,6 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   __shared__ double srho[LAST ? kNodeThreads : 1];
   __shared__ int sbad[LAST ? kNodeThreads : 1];
   __shared__ int s_halt;
-  __shared__ double s_sum[SEG && LAST ? kNodeThreads : 1];
-  __shared__ double s_rho[SEG && LAST ? kNodeThreads : 1];
-  __shared__ int s_bad[SEG && LAST ? kNodeThreads : 1];
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int32_t a_base = 0, b_base = 0, a_cnt = 0, b_cnt = 0;
   if (STAGE) {
@@ -674,7 +675,6 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
     for (int k = 0; k < 5; k++) Fa[k] = A.flux[5 * i + k];
   }
   if (threadIdx.x == 0) s_halt = A.st->halt;
-  if (SEG && LAST) { s_sum[threadIdx.x] = 0.0; s_rho[threadIdx.x] = 0.0; s_bad[threadIdx.x] = 0; }
   if (STAGE) cp_async_wait_all();
   __syncthreads();
   if (s_halt) return;  // block-uniform: the reduction below synchronises
@@ -929,17 +929,38 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   }
   if (!LAST || !A.level0) return;
   if (SEG) {
-    const int32_t m0 = A.mesh_id[(int64_t)blockIdx.x * blockDim.x];
+    // Nearly every block lies in one mesh: its norms are summed as a plain
+    // solver's are.  A block that spans meshes adds each node to its mesh's
+    // shared slot instead.  FP64 shared atomics are compare-and-swap loops, so
+    // 128 threads on one slot took longer than the rest of the stage: at 2.6M
+    // nodes in 16 meshes the last mixed stage ran 812 us with every block on
+    // that path against 262 us for the stages without norms; the V-cycle went
+    // from 2.04 to 1.53 ms (FP64, 12 meshes: 1.08 to 0.94 ms).
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x;
+    const int64_t i1 = i0 + blockDim.x < A.n ? i0 + blockDim.x : A.n;
+    const int32_t m0 = A.mesh_id[i0];
+    const int t = threadIdx.x;
+    if (A.mesh_id[i1 - 1] == m0) {  // block-uniform
+      if (block_sums(srms, srho, sbad, r2, rr, bad)) {
+        atomicAdd(A.seg_rms + m0, r2);
+        atomicAdd(A.seg_rho + m0, rr);
+        if (bad) atomicAdd(A.seg_bad + m0, bad);
+      }
+      return;
+    }
+    srms[t] = 0.0;
+    srho[t] = 0.0;
+    sbad[t] = 0;
+    __syncthreads();
     if (i < A.n) {
-      if (r2 != 0.0) atomicAdd(&s_sum[mid - m0], r2);
-      if (rr != 0.0) atomicAdd(&s_rho[mid - m0], rr);
-      if (bad) atomicAdd(&s_bad[mid - m0], bad);
+      if (r2 != 0.0) atomicAdd(&srms[mid - m0], r2);
+      if (rr != 0.0) atomicAdd(&srho[mid - m0], rr);
+      if (bad) atomicAdd(&sbad[mid - m0], bad);
     }
     __syncthreads();
-    const int t = threadIdx.x;
-    if (s_sum[t] != 0.0) atomicAdd(A.seg_rms + m0 + t, s_sum[t]);
-    if (s_rho[t] != 0.0) atomicAdd(A.seg_rho + m0 + t, s_rho[t]);
-    if (s_bad[t]) atomicAdd(A.seg_bad + m0 + t, s_bad[t]);
+    if (srms[t] != 0.0) atomicAdd(A.seg_rms + m0 + t, srms[t]);
+    if (srho[t] != 0.0) atomicAdd(A.seg_rho + m0 + t, srho[t]);
+    if (sbad[t]) atomicAdd(A.seg_bad + m0 + t, sbad[t]);
     return;
   }
   block_norms(srms, srho, sbad, r2, rr, bad, A.st);
