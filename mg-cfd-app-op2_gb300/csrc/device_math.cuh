@@ -24,10 +24,10 @@
 //     and the weight is kept as h = -w/2 so the central term needs no
 //     multiplication by -1/2 (exact: a power-of-two scaling).
 //
-// Every operation is an FP64 operation; all are IEEE-rounded except the two
-// square roots of node_prim (x * rsqrt(x), within about two ulp).  Results
-// differ from the reference only by rounding (relative 1e-16 per operation),
-// far inside the 1e-10 parity bar.
+// Every operation is an FP64 operation; all are IEEE-rounded except the
+// reciprocal and the two square roots of node_prim (within 0.501 ulp, see
+// rcp_fast).  Results differ from the reference only by rounding (relative
+// 1e-16 per operation), far inside the 1e-10 parity bar.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -45,26 +45,120 @@ struct NodePrim {
   double rinv;                   // 1 / rho
 };
 
-// sqrt(x) as x * rsqrt(x) for positive finite x: about 8 FMA-equivalents on
-// GB300 instead of about 10 for the correctly rounded square root, accurate
-// to about two ulp.  Zero, negative, infinite and NaN inputs (recognised from
-// the bit pattern on the integer pipe) take the IEEE square root, so the
-// special cases are exactly those of sqrt().
+// The 64-bit register of a double is packed and unpacked with PTX moves,
+// which the compiler cannot fold back into a floating-point conversion.
+__device__ __forceinline__ double pack_words(uint32_t hi, uint32_t lo) {
+  double d;
+  asm("mov.b64 %0, {%1, %2};" : "=d"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+
+__device__ __forceinline__ void unpack_words(double d, uint32_t& hi, uint32_t& lo) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(d));
+}
+
+// FP64 reciprocal, quotient and square root with most of the work on the
+// FP32 and integer pipes.
+//
+// The FP64 pipe bounds every FP64 node kernel here, and the compiler's
+// 1.0 / x, a / b and sqrt(x) each issue 7 to 10 operations on it.  These
+// take an FP32 approximation, refine it in FP32 to a pair h + l within about
+// 2^-43 of the result (one Newton step whose residual is formed exactly by
+// FMA), put the pair's bits together as one binary64 number on the integer
+// pipe, and finish with one Newton step in FP64:
+//   reciprocal  y + y (1 - x y)                   2 FP64 operations
+//   quotient    q + y (a - b q),  q = a y         3
+//   square root s + (x - s s) / (2 s)             2
+// The residual is one FMA, so the error before the last rounding is the
+// square of the seed's (2^-86); for the root, whose 1/(2s) is the FP32 one,
+// 2^-43 * 2^-21.  Results are within 0.5 + 2^-30 (root: 0.5 + 2^-10) units in
+// the last place.  Positive arguments in [2^-60, 2^60) only, recognised from the
+// exponent; everything else (zero, negative, huge, tiny, infinite, NaN) takes
+// the IEEE operation.  Measured: the 200^3 FP64 solve (25 V-cycles) 207 ->
+// 197 ms, 12 batched FP64 meshes 18.7 -> 17.4 ms, the per-loop V-cycles at
+// 100^3 6.40 -> 5.94 ms.
+constexpr uint32_t kSeedLo = (1023u - 60u) << 20, kSeedSpan = 120u << 20;
+
+__device__ __forceinline__ bool seedable(uint32_t hi) { return hi - kSeedLo < kSeedSpan; }
+
+// x = h + l, h its leading 24 bits, l the rest to FP32 accuracy.
+__device__ __forceinline__ void seed_split(uint32_t hi, uint32_t lo, float& h, float& l) {
+  h = __uint_as_float(((hi - (896u << 20)) << 3) | (lo >> 29));
+  l = __fmul_rn(__uint2float_rn(lo & 0x1fffffffu), __uint_as_float(((hi >> 20) - 948u) << 23));  // * 2^(e - 52)
+}
+
+// The binary64 number nearest h + l for normal positive h and |l| <= 2^-20 h,
+// on the integer pipe.  After renormalising (Dekker's Fast2Sum) l is at most
+// half a unit in the last place of h, so counting it in units of the last
+// place of h's binary64 pattern crosses no power of two -- except below
+// h = 2^k with l < 0, where the patterns are half as far apart.
+__device__ __forceinline__ double seed_join(float a, float b) {
+  const float h = __fadd_rn(a, b);
+  const float l = __fsub_rn(b, __fsub_rn(h, a));
+  const uint32_t u = __float_as_uint(h);
+  const uint32_t below = ((u & 0x7fffffu) == 0u && l < 0.0f) ? 1u : 0u;
+  const int delta = __float2int_rn(__fmul_rn(l, __uint_as_float((306u - (u >> 23) + below) << 23)));  // l / 2^(e - 52)
+  const unsigned long long base = ((unsigned long long)((u >> 3) + (896u << 20)) << 32) | (u << 29);
+  return __longlong_as_double((long long)(base + (unsigned long long)(long long)delta));
+}
+
+// 1/x to about 2^-44.
+__device__ __forceinline__ double rcp_seed(uint32_t hi, uint32_t lo) {
+  float h, l, y;
+  seed_split(hi, lo, h, l);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(h));
+  const float e = __fmaf_rn(-l, y, __fmaf_rn(-h, y, 1.0f));
+  return seed_join(y, __fmul_rn(y, e));
+}
+
+static __device__ __noinline__ double rcp_ieee(double x) { return 1.0 / x; }
+static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
+static __device__ __noinline__ double sqrt_ieee(double x) { return sqrt(x); }
+
+__device__ __forceinline__ double rcp_fast(double x) {
+  uint32_t hi, lo;
+  unpack_words(x, hi, lo);
+  if (!seedable(hi)) return rcp_ieee(x);
+  const double y = rcp_seed(hi, lo);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// a / b, for |a| in [2^-900, 2^900) and b as above.
+__device__ __forceinline__ double div_fast(double a, double b) {
+  uint32_t ahi, alo, hi, lo;
+  unpack_words(a, ahi, alo);
+  unpack_words(b, hi, lo);
+  if (!seedable(hi) || (ahi & 0x7fffffffu) - ((1023u - 900u) << 20) >= (1800u << 20)) return div_ieee(a, b);
+  const double y = rcp_seed(hi, lo);
+  const double q = a * y;
+  return fma(fma(-q, b, a), y, q);
+}
+
 __device__ __forceinline__ double sqrt_fast(double x) {
-  const long long b = __double_as_longlong(x);
-  return (b > 0 && b < 0x7ff0000000000000ll) ? x * rsqrt(x) : sqrt(x);
+  uint32_t hi, lo;
+  unpack_words(x, hi, lo);
+  if (!seedable(hi)) return sqrt_ieee(x);
+  float h, l, y;
+  seed_split(hi, lo, h, l);
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(h));
+  const float s0 = __fmul_rn(h, y), g = __fmul_rn(0.5f, y);
+  const float p = __fmul_rn(s0, s0);
+  const float r = __fadd_rn(__fsub_rn(__fsub_rn(h, p), __fmaf_rn(s0, s0, -p)), l);  // x - s0^2
+  const double s = seed_join(s0, __fmul_rn(r, g));
+  const uint32_t u = __float_as_uint(g);
+  return fma(fma(-s, s, x), pack_words((u >> 3) + (896u << 20), u << 29), s);
 }
 
 // inlined_funcs.h:98-130 with one reciprocal instead of three divisions, and
 // without forming the velocity: with m2 = |m|^2,
 //   rho |u|^2 = m2 / rho,   |u| = sqrt(m2) / rho,
 // so p = (gamma - 1)(rhoE - m2/(2 rho)) and |u| = sqrt(m2) * (1/rho) take
-// five FP64 operations fewer than u = m/rho, |u|^2 = u.u (about 33 FMA
-// equivalents per node instead of 35).
+// five FP64 operations fewer than u = m/rho, |u|^2 = u.u.  15 FP64 operations
+// per node (33 with the compiler's reciprocal and reciprocal square roots).
 __device__ __forceinline__ NodePrim node_prim(double rho, double mx, double my, double mz, double rhoE) {
   NodePrim n;
   n.rho = rho; n.mx = mx; n.my = my; n.mz = mz; n.rhoE = rhoE;
-  n.rinv = 1.0 / rho;
+  n.rinv = rcp_fast(rho);
   const double m2 = fma(mz, mz, fma(my, my, mx * mx));
   n.p = kGammaM1 * fma(-0.5 * m2, n.rinv, rhoE);
   n.s = sqrt_fast(m2) * n.rinv + sqrt_fast(kGammaD * n.p * n.rinv);
@@ -133,18 +227,6 @@ __device__ __forceinline__ void farfield_flux(const NodePrim& b, double wx, doub
 //             overflow rounds to infinity, NaNs keep the top payload bits and
 //             become quiet; results in the binary32 subnormal range are
 //             rounded with the same rule from the full 53-bit significand.
-// The 64-bit register is packed and unpacked with PTX moves, which the
-// compiler cannot fold back into a floating-point conversion.
-__device__ __forceinline__ double pack_words(uint32_t hi, uint32_t lo) {
-  double d;
-  asm("mov.b64 %0, {%1, %2};" : "=d"(d) : "r"(lo), "r"(hi));
-  return d;
-}
-
-__device__ __forceinline__ void unpack_words(double d, uint32_t& hi, uint32_t& lo) {
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(d));
-}
-
 // Zero, subnormal, infinity and NaN inputs: a separate, rarely taken call, so
 // the common path issues only its own integer instructions.  A subnormal is
 // first scaled by 2^24 in FP32 (exact) and its exponent corrected after.

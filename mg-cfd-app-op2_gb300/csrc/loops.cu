@@ -103,7 +103,7 @@ __global__ void k_calculate_dt(int32_t n, const double* __restrict__ var, const 
   MGCFD_GRID_STRIDE(i, n) {
     const double* x = var + 5 * i;
     NodePrim p = node_prim(x[0], x[1], x[2], x[3], x[4]);
-    dt[i] = 0.5 * (cbrt(vol[i]) / p.s);
+    dt[i] = 0.5 * div_fast(cbrt(vol[i]), p.s);
   }
 }
 
@@ -141,7 +141,7 @@ __global__ void k_min_dt(int32_t n, const double* __restrict__ dt, double* __res
 __global__ void k_step_factor(int32_t n, const double* __restrict__ vol, const double* __restrict__ min_dt,
                               double* __restrict__ sf) {
   const double m = *min_dt;
-  MGCFD_GRID_STRIDE(i, n) sf[i] = m / vol[i];
+  MGCFD_GRID_STRIDE(i, n) sf[i] = div_fast(m, vol[i]);
 }
 
 // flux.h:41-208 over edges with atomic increments at both ends.

@@ -861,7 +861,7 @@ __global__ void k_plan_calculate_dt(int32_t n, const double* __restrict__ var, c
     }
     const double* x = var + 5 * i;
     const NodePrim p = node_prim(x[0], x[1], x[2], x[3], x[4]);
-    dt[i] = 0.5 * (c / p.s);
+    dt[i] = 0.5 * div_fast(c, p.s);
   }
 }
 

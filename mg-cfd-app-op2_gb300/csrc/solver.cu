@@ -226,7 +226,7 @@ __device__ __forceinline__ void step_begin_core(int64_t i, bool live, const doub
         sp = p.s;
       }
       cv = cbrt_vol[i];
-      if (SEG) key = dt_candidate_key(0.5 * (cv / sp));  // time_stepping_kernels.h:31
+      if (SEG) key = dt_candidate_key(0.5 * div_fast(cv, sp));  // time_stepping_kernels.h:31
       else est = 0.5f * __fdividef(d2f_bits(cv), d2f_bits(sp));
     }
   }
@@ -247,7 +247,7 @@ __device__ __forceinline__ void step_begin_core(int64_t i, bool live, const doub
     for (int w = 1; w < kNodeThreads / 32; w++) bk = min(bk, sest[w]);
     const float m32 = bk == 0xffffffffu ? INFINITY : fkey_inv(bk);
     if (live && (!normal || est <= m32 + fabsf(m32) * 4e-6f))
-      key = dt_candidate_key(0.5 * (cv / sp));  // time_stepping_kernels.h:31
+      key = dt_candidate_key(0.5 * div_fast(cv, sp));  // time_stepping_kernels.h:31
   }
   if (SEG) {
     const int32_t m0 = mesh_id[(int64_t)blockIdx.x * blockDim.x];

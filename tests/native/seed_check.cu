@@ -1,0 +1,36 @@
+// Test harness (not part of the library): the FP64 reciprocal, quotient and
+// square root with FP32 seeds of device_math.cuh on host arrays.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "device_math.cuh"
+
+namespace {
+
+__global__ void k_check(int64_t n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ r,
+                        double* __restrict__ q, double* __restrict__ s) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  r[i] = mgcfd::rcp_fast(b[i]);
+  q[i] = mgcfd::div_fast(a[i], b[i]);
+  s[i] = mgcfd::sqrt_fast(b[i]);
+}
+
+}  // namespace
+
+// Host buffers in (a, b) and out (1/b, a/b, sqrt(b)); returns a cudaError_t value.
+extern "C" int seed_check(int64_t n, const double* a, const double* b, double* r, double* q, double* s) {
+  const size_t bytes = sizeof(double) * (size_t)n;
+  double* d = nullptr;
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&d), 5 * bytes);
+  if (e) return (int)e;
+  if (!(e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice)) &&
+      !(e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice))) {
+    k_check<<<(unsigned)((n + 127) / 128), 128>>>(n, d, d + n, d + 2 * n, d + 3 * n, d + 4 * n);
+    if (!(e = cudaGetLastError()) && !(e = cudaMemcpy(r, d + 2 * n, bytes, cudaMemcpyDeviceToHost)) &&
+        !(e = cudaMemcpy(q, d + 3 * n, bytes, cudaMemcpyDeviceToHost)))
+      e = cudaMemcpy(s, d + 4 * n, bytes, cudaMemcpyDeviceToHost);
+  }
+  cudaFree(d);
+  return (int)e;
+}

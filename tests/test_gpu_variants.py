@@ -1,9 +1,14 @@
 """Kernel variants chosen by a rule on sizes, at the sizes where the rule or
 the variant can go wrong (GPU)."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 
 import mgcfd
+from mgcfd import _build
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +36,82 @@ def test_batch_norms_blocks_within_and_across_meshes(precision, axes):
         np.testing.assert_allclose([brms, brho], [rms, rho], rtol=1e-6, atol=0)
         solo.close()
     batch.close()
+
+
+def _ulps(x, exact):
+    """|x - exact| in units of the last place of exact (exact: long double)."""
+    _, e = np.frexp(exact.astype(np.float64))
+    return np.abs(x.astype(np.longdouble) - exact) * np.ldexp(np.longdouble(1), 53 - e)
+
+
+def _seed_inputs(kind):
+    rng = np.random.default_rng(11)
+    n = 400_000
+    if kind == "mantissas":  # every exponent of the fast range and beyond its ends
+        b = np.ldexp(1.0 + rng.random(n), rng.integers(-64, 64, n))
+    elif kind == "near_powers":  # a few units around every power of two, and around FP32 rounding ties
+        k = rng.integers(-61, 62, n)
+        b = np.ldexp(1.0, k) * (1.0 + rng.integers(-40, 41, n) * 2.0 ** -53)
+        tie = rng.random(n) < 0.5
+        f = rng.integers(0, 1 << 23, n) * 2.0 ** -23 + 2.0 ** -24
+        b = np.where(tie, np.ldexp(1.0 + f, k) * (1.0 + rng.integers(-3, 4, n) * 2.0 ** -52), b)
+    else:  # results next to a power of two, from both sides
+        k = rng.integers(-59, 60, n)
+        r = np.ldexp(1.0, k // 2) * (1.0 + rng.integers(-2000, 2001, n) * 2.0 ** -rng.integers(22, 53, n))
+        b = np.where(rng.random(n) < 0.5, 1.0 / r, r * r)
+    a = np.ldexp(1.0 + rng.random(n), rng.integers(-300, 300, n)) * rng.choice([-1.0, 1.0], n)
+    return a, b
+
+
+@pytest.fixture(scope="module")
+def seed_check():
+    here = Path(__file__).resolve().parent
+    out = here / "_build" / "libseed_check.so"
+    out.parent.mkdir(exist_ok=True)
+    subprocess.run([_build._nvcc(), *_build.ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
+                    f"-I{_build.CSRC}", str(here / "native" / "seed_check.cu"), "-o", str(out)], check=True,
+                   capture_output=True)
+    lib = C.CDLL(str(out))
+
+    def run(a, b):
+        outs = [np.empty(len(b)) for _ in range(3)]
+        p = [x.ctypes.data_as(C.c_void_p) for x in (a, b, *outs)]
+        assert lib.seed_check(C.c_int64(len(b)), *p) == 0
+        return outs
+
+    return run
+
+
+@pytest.mark.parametrize("kind", ["mantissas", "near_powers", "near_power_results"])
+def test_seeded_reciprocal_quotient_root(seed_check, kind):
+    """rcp_fast, div_fast and sqrt_fast against long double.  The seeds are
+    within 2^-42, so one Newton step leaves 0.5 ulp of rounding and, for the
+    root, 2^-42 * 2^-21 * 2^53 = 2^-10 ulp more: 0.5 + 2^-9 is the bound."""
+    a, b = _seed_inputs(kind)
+    r, q, s = seed_check(a, b)
+    A, B = a.astype(np.longdouble), b.astype(np.longdouble)
+    slack = 0.5 + 2.0 ** -9
+    assert _ulps(r, 1 / B).max() <= slack
+    assert _ulps(q, A / B).max() <= slack
+    assert _ulps(s, np.sqrt(B)).max() <= slack
+
+
+def test_seeded_forms_keep_the_ieee_special_cases(seed_check):
+    """Operands outside the fast range give the IEEE result bit for bit; the
+    ones just inside it (2^-60 and the number below 2^60, whose reciprocal and
+    root lie 2^-53 ulp from a rounding tie) are held to the bound above."""
+    edge = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 2.2e-308, 1.7e308, -1.0, -4.0, 2.0 ** -60,
+                     2.0 ** 60, np.nextafter(2.0 ** 60, 0), np.nextafter(2.0 ** -60, 0), 2.0 ** -61, 1e-200, 1e200])
+    a, b = (x.ravel().copy() for x in np.meshgrid(edge, edge))
+    r, q, s = seed_check(a, b)
+    fast_b = (b >= 2.0 ** -60) & (b < 2.0 ** 60)
+    fast_q = fast_b & (np.abs(a) >= 2.0 ** -900) & (np.abs(a) < 2.0 ** 900)
+    with np.errstate(all="ignore"):
+        want = [1.0 / b, a / b, np.sqrt(b)]
+        exact = [1 / b.astype(np.longdouble), a.astype(np.longdouble) / b, np.sqrt(b.astype(np.longdouble))]
+    for got, w, ld, fast in zip((r, q, s), want, exact, (fast_b, fast_q, fast_b)):
+        nan = np.isnan(w)
+        assert np.isnan(got[nan]).all()
+        ieee = ~nan & ~fast
+        assert np.array_equal(got[ieee].view(np.uint64), w[ieee].view(np.uint64))
+        assert _ulps(got[fast], ld[fast]).max() <= 0.5 + 2.0 ** -9
