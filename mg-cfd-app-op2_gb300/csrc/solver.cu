@@ -20,7 +20,6 @@
 //   ch_off/ch_list: restriction children of each coarse node
 //
 // Kernels per smoothing step (euler3d.cpp:467-550):
-//   memset(min_dt key)                      get_min_dt's DBL_MAX start
 //   k_step_begin   nodes  old = var, primitives, dt, block min -> atomicMin
 //                         (a step that a prolongation precedes -- every
 //                         level-0 step after the first -- begins inside
@@ -35,8 +34,23 @@
 //   plain multi-level solver takes the level-0 rms and NaN/Inf count in the
 //   restriction that follows instead of the last stage)
 // then k_restrict (coarse nodes, children mean, mg.h:29-64) or k_prolong
-// (fine nodes, mg.h:66-88), and under a stop rule k_cycle_end after each
-// V-cycle.
+// (fine nodes, mg.h:66-88), which also reset the min_dt key of the level just
+// smoothed (get_min_dt's DBL_MAX start), and under a stop rule k_cycle_end
+// after each V-cycle.
+//
+// These launches follow one another as programmatic dependents: each loads
+// what set-up left constant (ids, weights, offsets, volumes), then waits for
+// the kernel before it (grid_wait).  A wait returns when the whole grid
+// before it has finished and its writes are visible, so the order is the
+// stream's; what overlaps is the launch and the constant loads with the
+// previous kernel's end.  Kernels let the next one start when their blocks
+// exit, the fused stages before their last stores (grid_trigger): started any
+// earlier, its blocks fill the slots that happen to be free and sit unevenly
+// on the SMs (48^3, DW: 218 us per V-cycle when triggered at the start, 160
+// like this, 195 with plain launches, memsets and copies between them).  Data
+// that a kernel of the chain writes is read after the wait, through pointers
+// without __restrict__ (a load from a const __restrict__ pointer may be
+// hoisted above it or go through the read-only path).
 //
 // Failure handling: min_dt < 0 and NaN/Inf at level 0 set a sticky device
 // status word; every later kernel sees it and returns, so the run stops at the
@@ -79,6 +93,42 @@ void keep_freed_memory(int dev) {
 
 // ---------------------------------------------------------------------------
 // Kernels.
+
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launches a kernel that begins with grid_wait as the programmatic dependent
+// of the kernel before it in the stream (`chained`), else in plain stream order.
+template <class... P, class... A>
+void launch(void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t stream, bool chained, A... args) {
+  cudaLaunchConfig_t c = {};
+  cudaLaunchAttribute at;
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = stream;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, P(args)...);  // errors: the callers' cudaGetLastError
+}
+
+// The min_dt keys of the level just smoothed: kept as the ones its last step
+// used (for the step factors that a fetch reports), then reset for its next
+// step.  Run by one block of the transfer that follows the step.
+struct KeyReset {
+  unsigned long long* key;
+  unsigned long long* used;
+  int32_t count;  // one key per mesh of a batch
+};
+
+__device__ __forceinline__ void reset_keys(const KeyReset& K, bool halted) {
+  if (blockIdx.x != 0) return;
+  for (int32_t t = threadIdx.x; t < K.count; t += blockDim.x) {
+    K.used[t] = K.key[t];
+    if (!halted) K.key[t] = ~0ull;
+  }
+}
 
 __device__ __forceinline__ void store_rec(double* rec, int64_t i, const NodePrim& p) {
   double4_32a* r = reinterpret_cast<double4_32a*>(rec + 8 * i);
@@ -190,11 +240,9 @@ __global__ void k_init_state(int32_t n, double* __restrict__ rec, double v0, dou
 // primitives go to rec2 as pairs (the edge flux's inputs); rec keeps the
 // state only.
 template <bool MIXED, bool SEG, bool DW>
-__device__ __forceinline__ void step_begin_core(int64_t i, bool live, const double x[5], double* __restrict__ rec,
-                                                double* __restrict__ rec2, float* __restrict__ rec32,
-                                                double* __restrict__ old, const double* __restrict__ cbrt_vol,
-                                                unsigned long long* __restrict__ dt_key,
-                                                const int32_t* __restrict__ mesh_id) {
+__device__ __forceinline__ void step_begin_core(int64_t i, bool live, const double x[5], double* rec, double* rec2,
+                                                float* rec32, double* old, const double* __restrict__ cbrt_vol,
+                                                unsigned long long* dt_key, const int32_t* __restrict__ mesh_id) {
   __shared__ unsigned long long smin[kNodeThreads / 32];
   __shared__ unsigned int sest[kNodeThreads / 32];
   __shared__ unsigned long long s_key[SEG ? kNodeThreads : 1];
@@ -271,27 +319,25 @@ __device__ __forceinline__ void step_begin_core(int64_t i, bool live, const doub
 
 // The step begin on its own (a step that no prolongation precedes).
 template <bool MIXED, bool SEG, bool DW = false>
-__global__ void __launch_bounds__(kNodeThreads) k_step_begin(int32_t n, double* __restrict__ rec,
-                                                             double* __restrict__ rec2,
-                                                             float* __restrict__ rec32, double* __restrict__ old,
-                                                             const double* __restrict__ cbrt_vol,
-                                                             unsigned long long* __restrict__ dt_key,
-                                                             const DevStatus* __restrict__ st,
+__global__ void __launch_bounds__(kNodeThreads) k_step_begin(int32_t n, double* rec, double* rec2, float* rec32,
+                                                             double* old, const double* __restrict__ cbrt_vol,
+                                                             unsigned long long* dt_key, const DevStatus* st,
                                                              const int32_t* __restrict__ mesh_id,
-                                                             const SegStop* __restrict__ seg_stop) {
+                                                             const SegStop* seg_stop) {
   __shared__ int s_halt;
-  if (threadIdx.x == 0) s_halt = st->halt;
-  __syncthreads();
-  if (s_halt) return;  // block-uniform: the reduction below synchronises
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  // Batched solvers under a stop rule: a stopped mesh's nodes change no more.
-  const bool live = i < n && !(SEG && seg_stop && seg_stop[mesh_id[i]].halt);
+  grid_wait();
   double x[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (live) {
+  if (i < n) {
     const double4_32a* r = reinterpret_cast<const double4_32a*>(rec + 8 * i);
     const double4_32a v = r[0];
     x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; x[4] = r[1].x;
   }
+  if (threadIdx.x == 0) s_halt = st->halt;
+  __syncthreads();
+  if (s_halt) return;  // block-uniform: the reduction below synchronises
+  // Batched solvers under a stop rule: a stopped mesh's nodes change no more.
+  const bool live = i < n && !(SEG && seg_stop && seg_stop[mesh_id[i]].halt);
   step_begin_core<MIXED, SEG, DW>(i, live, x, rec, rec2, rec32, old, cbrt_vol, dt_key, mesh_id);
 }
 
@@ -299,15 +345,16 @@ __global__ void __launch_bounds__(kNodeThreads) k_step_begin(int32_t n, double* 
 // (GATHER=false) or stored per edge for the node-side gather (GATHER=true).
 template <bool GATHER>
 __global__ void k_flux_f64(int32_t ne, const int2* __restrict__ e2n, const double4_32a* __restrict__ w4,
-                           const double* __restrict__ rec, double* __restrict__ flux, double* __restrict__ fe,
-                           const DevStatus* __restrict__ st) {
-  if (st->halt) return;
+                           const double* rec, double* flux, double* fe,
+                           const DevStatus* st) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const int2 ab = e2n[e];
-  const double4_32a w = w4[e];
+  const bool live = e < ne;
+  const int2 ab = live ? e2n[e] : make_int2(0, 0);
+  const double4_32a w = w4[live ? e : 0];  // (launched for ne > 0 only)
+  grid_wait();
   const NodePrim a = load_rec(rec, ab.x);
   const NodePrim b = load_rec(rec, ab.y);
+  if (!live || st->halt) return;
   double f[5];
   edge_flux(a, b, w.x, w.y, w.z, w.w, f);
   if (GATHER) {
@@ -330,15 +377,16 @@ __global__ void k_flux_f64(int32_t ne, const int2* __restrict__ e2n, const doubl
 // increments in binary64, by FP64 atomics or stored per edge as k_flux_f64.
 template <bool GATHER>
 __global__ void k_flux_dw(int32_t ne, const int2* __restrict__ e2n, const double4_32a* __restrict__ w2,
-                          const double* __restrict__ rec2, double* __restrict__ flux, double* __restrict__ fe,
-                          const DevStatus* __restrict__ st) {
-  if (st->halt) return;
+                          const double* rec2, double* flux, double* fe,
+                          const DevStatus* st) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const int2 ab = e2n[e];
-  const double4_32a w = w2[e];
+  const bool live = e < ne;
+  const int2 ab = live ? e2n[e] : make_int2(0, 0);
+  const double4_32a w = w2[live ? e : 0];  // (launched for ne > 0 only)
+  grid_wait();
   const NodePrimDW a = load_prim_dw(rec2, ab.x);
   const NodePrimDW b = load_prim_dw(rec2, ab.y);
+  if (!live || st->halt) return;
   double f[5];
   edge_flux_dw(a, b, dw_unpack(w.x), dw_unpack(w.y), dw_unpack(w.z), dw_unpack(w.w), f);
   if (GATHER) {
@@ -437,15 +485,16 @@ __global__ void k_gather_edges(int32_t ne, const int32_t* __restrict__ idx, cons
 // here and adds them with FP64 atomics.
 template <bool GATHER>
 __global__ void k_flux_mixed(int32_t ne, const int2* __restrict__ e2n, const float4* __restrict__ w4f,
-                             const float* __restrict__ rec32, double* __restrict__ flux, float* __restrict__ fe32,
-                             const DevStatus* __restrict__ st) {
-  if (st->halt) return;
+                             const float* rec32, double* flux, float* fe32,
+                             const DevStatus* st) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const int2 ab = e2n[e];
-  const float4 w = w4f[e];
+  const bool live = e < ne;
+  const int2 ab = live ? e2n[e] : make_int2(0, 0);
+  const float4 w = w4f[live ? e : 0];  // (launched for ne > 0 only)
+  grid_wait();
   const NodePrimF a = load_rec32(rec32, ab.x);
   const NodePrimF b = load_rec32(rec32, ab.y);
+  if (!live || st->halt) return;
   float f[5];
   edge_flux_f32(a, b, w, f);
   if (GATHER) {
@@ -494,7 +543,8 @@ __global__ void k_stream(int32_t ne, const int2* __restrict__ e2n, const double4
 struct UpdateArgs {
   int32_t n;
   int32_t level0;
-  double inv_div;  // 1 / (RK + 1 - rk)
+  int32_t clear_norms;  // first stage at level 0: the number of norm accumulators to clear, else 0
+  double inv_div;       // 1 / (RK + 1 - rk)
   double* rec;
   double* rec2;            // DW: the next stage's primitives as pairs
   const double* rec2_in;   // DW fused: the stage's input primitives
@@ -662,19 +712,38 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
     for (int t = threadIdx.x; t < a_cnt; t += blockDim.x) cp_async4(s_aid + t, &A.e2n[a_base + t].y);
     for (int t = threadIdx.x; t < b_cnt; t += blockDim.x) cp_async4(s_bid + t, A.b_nbr + b_base + t);
   }
-  // The node's own data is loaded before the block-uniform halt and min_dt
-  // checks so that its latency overlaps them; nothing is written before.
+  // Constant tables before the wait; then the node's own data before the
+  // block-uniform halt and min_dt checks, so that its latency overlaps them;
+  // nothing is written before.
   double o[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, Fa[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, ivol = 0.0;
   int32_t bi = -1;
+  EdgeRange er{0, 0, 0, 0};
+  int32_t k0 = 0, k1 = 0;  // DW fused: the node's entries
   if (!GATHER && i < A.n) {  // (the gather forms load them after their edge loop)
-#pragma unroll
-    for (int k = 0; k < 5; k++) o[k] = A.old[5 * i + k];
     ivol = A.inv_vol[i];
     bi = A.bidx[i];
+  } else if (FUSED && DW && i < A.n) {
+    k0 = A.off2[i];
+    k1 = A.off2[i + 1];
+  } else if (GATHER && !EP && i < A.n) {
+    er = edge_range(A, i);
+  }
+  grid_wait();
+  if (!GATHER && i < A.n) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) o[k] = A.old[5 * i + k];
 #pragma unroll
     for (int k = 0; k < 5; k++) Fa[k] = A.flux[5 * i + k];
   }
   if (threadIdx.x == 0) s_halt = A.st->halt;
+  if (A.clear_norms && blockIdx.x == 0) {  // this step's norms start from zero
+    if (SEG) {
+      for (int32_t t = threadIdx.x; t < A.clear_norms; t += blockDim.x) { A.seg_rms[t] = 0.0; A.seg_rho[t] = 0.0; }
+    } else if (threadIdx.x == 0) {
+      A.st->rms_acc = 0.0;
+      A.st->rho_acc = 0.0;
+    }
+  }
   if (STAGE) cp_async_wait_all();
   __syncthreads();
   if (s_halt) return;  // block-uniform: the reduction below synchronises
@@ -772,7 +841,6 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
       const dwf s_me = dw_unpack(A.rec2_in[8 * i + 6]);
       NodeFluxDW acc;
       node_flux_dw_init(acc);
-      const int32_t k0 = A.off2[i], k1 = A.off2[i + 1];
       int2 next = k0 < k1 ? A.ent2[k0] : make_int2(0, 0);
       for (int32_t j = k0; j < k1; j++) {
         const int2 en = next;  // the following entry loads during this edge's arithmetic
@@ -796,7 +864,6 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
 #pragma unroll
       for (int k = 0; k < 5; k++) F[k] = 0.0;
       float f[5];
-      const EdgeRange er = edge_range(A, i);
       for (int32_t j = 0; j < er.deg; j++) {
         const bool end_a = j < er.na;
         const int32_t ja = end_a ? er.a0 + j : 0, jb = end_a ? 0 : er.b0 + j - er.na;  // both in range
@@ -827,7 +894,6 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
       // Unevaluated FP32 pairs (hi, lo) fed by error-free TwoSum steps;
       // one FP64 add per variable at the end.
       float hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-      const EdgeRange er = edge_range(A, i);
       for (int32_t j = 0; j < er.deg; j++) {
         const bool end_a = j < er.na;
         const int64_t e = end_a ? er.a0 + j : A.b_list[end_a ? 0 : er.b0 + j - er.na];
@@ -842,7 +908,6 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
     } else if (GATHER) {
 #pragma unroll
       for (int k = 0; k < 5; k++) F[k] = 0.0;
-      const EdgeRange er = edge_range(A, i);
       for (int32_t j = 0; j < er.deg; j++) {
         const bool end_a = j < er.na;
         const int64_t e = end_a ? er.a0 + j : A.b_list[end_a ? 0 : er.b0 + j - er.na];
@@ -879,6 +944,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
       }
       add_boundary(p, A.bdata + 12 * (int64_t)bi, F);
     }
+    if (FUSED) grid_trigger();
     const double factor = (min_dt * ivol) * A.inv_div;  // step_factor / (RK+1-rk)
     double v[5];
 #pragma unroll
@@ -975,27 +1041,32 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
 // kernel would run.
 template <bool NORMS>
 __global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int32_t* __restrict__ ch_off,
-                                                           const int32_t* __restrict__ ch_list,
-                                                           const double* __restrict__ frec, double* __restrict__ crec,
-                                                           const double* __restrict__ fres, DevStatus* st,
+                                                           const int32_t* __restrict__ ch_list, const double* frec,
+                                                           double* crec, const double* fres, DevStatus* st,
                                                            const int32_t* __restrict__ mesh_id,
-                                                           const SegStop* __restrict__ seg_stop) {
+                                                           const SegStop* seg_stop, KeyReset fine_keys) {
   __shared__ double srms[NORMS ? kNodeThreads : 1], srho[NORMS ? kNodeThreads : 1];
   __shared__ int sbad[NORMS ? kNodeThreads : 1];
-  __shared__ int s_halt;
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t lo = c < nc ? ch_off[c] : 0, hi = c < nc ? ch_off[c + 1] : 0;
+  grid_wait();
+  // The same for every thread of the launch, except that the norms' blocks
+  // may set it: one thread reads it for its block, whose reduction synchronises.
+  int halted;
   if (NORMS) {
+    __shared__ int s_halt;
     if (threadIdx.x == 0) s_halt = st->halt;
     __syncthreads();
-    if (s_halt) return;  // block-uniform: the reduction below synchronises
-  } else if (st->halt) {
-    return;
+    halted = s_halt;
+  } else {
+    halted = st->halt;
   }
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  reset_keys(fine_keys, halted);
+  if (halted) return;
   double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sums of squared residuals, one chain per variable
   int bad = 0;
-  const int32_t lo = c < nc ? ch_off[c] : 0, hi = c < nc ? ch_off[c + 1] : 0;
-  const bool halted = c < nc && seg_stop && seg_stop[mesh_id[c]].halt;  // a stopped mesh of a batch
-  if (hi > lo && !halted) {  // no children: state unchanged (avg = 1 on untouched values)
+  const bool stopped = c < nc && seg_stop && seg_stop[mesh_id[c]].halt;  // a stopped mesh of a batch
+  if (hi > lo && !stopped) {  // no children: state unchanged (avg = 1 on untouched values)
     double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     for (int32_t j = lo; j < hi; j++) {
       const int64_t f = ch_list[j];
@@ -1037,19 +1108,24 @@ struct BeginArgs {
 // the level's state again; every thread reaches the block reduction.
 template <bool BEGIN, bool MIXED, bool SEG, bool DW>
 __global__ void __launch_bounds__(kNodeThreads) k_prolong(int32_t nf, const int32_t* __restrict__ n2mg,
-                                                          const double4_32a* __restrict__ dvec,
-                                                          double* __restrict__ frec, const double* __restrict__ fres,
-                                                          const double* __restrict__ cres,
-                                                          const DevStatus* __restrict__ st,
+                                                          const double4_32a* __restrict__ dvec, double* frec,
+                                                          const double* fres, const double* cres, const DevStatus* st,
                                                           const int32_t* __restrict__ mesh_id,
-                                                          const SegStop* __restrict__ seg_stop, BeginArgs B) {
-  if (st->halt) return;  // the same for every thread of the launch
+                                                          const SegStop* seg_stop, BeginArgs B, KeyReset coarse_keys) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int64_t c = 0;
+  double4_32a d = make_double4_32a(0.0, 0.0, 0.0, 0.0);
+  if (i < nf) {
+    c = n2mg[i];
+    d = dvec[i];
+  }
+  grid_wait();
+  const int halted = st->halt;  // the same for every thread of the launch
+  reset_keys(coarse_keys, halted);
+  if (halted) return;
   const bool live = i < nf && !(seg_stop && seg_stop[mesh_id[i]].halt);  // not a stopped mesh of a batch
   double x[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   if (live) {
-    const int64_t c = n2mg[i];
-    const double4_32a d = dvec[i];
     // The record's first four values as one 32-byte access, the fifth alone.
     double4_32a* r4 = reinterpret_cast<double4_32a*>(frec + 8 * i);
     double4_32a v = r4[0];
@@ -1098,6 +1174,7 @@ __global__ void k_bside(int32_t ne, const int32_t* __restrict__ b_list, const in
 // residual norm sqrt(sum(res_rho^2) / N0) and stop further work (not an
 // error) when the rule is met.  One thread.
 __global__ void k_cycle_end(DevStatus* st, double n0, int32_t max_cycles, double drop) {
+  grid_wait();
   if (st->halt) return;
   const int c = ++st->cycles_done;
   const double rho = sqrt(st->rho_acc / n0);
@@ -1111,10 +1188,10 @@ __global__ void k_cycle_end(DevStatus* st, double n0, int32_t max_cycles, double
 
 // The same per mesh of a batched solver, one thread per mesh: a mesh that
 // met the rule, or failed (min_dt < 0, NaN/Inf), stops changing.
-__global__ void k_cycle_end_seg(int32_t nseg, SegStop* __restrict__ ss, const double* __restrict__ seg_rho,
-                                const double* __restrict__ n0, const int* __restrict__ seg_neg,
-                                const int* __restrict__ seg_bad, int32_t max_cycles, double drop) {
+__global__ void k_cycle_end_seg(int32_t nseg, SegStop* ss, const double* seg_rho, const double* __restrict__ n0,
+                                const int* seg_neg, const int* seg_bad, int32_t max_cycles, double drop) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  grid_wait();
   if (m >= nseg || ss[m].halt) return;
   if (seg_neg[m] || seg_bad[m]) {
     ss[m].halt = 1;
@@ -1165,10 +1242,10 @@ int edge_threads(const mgcfd_solver* s) { return s->opt.block_size > 0 ? s->opt.
 
 // Launchers indexed by the kernels' compile-time variants.
 template <bool G, bool L, bool M, bool S>
-void launch_update(int grid_n, cudaStream_t st, const UpdateArgs& A) {
-  k_update<G, L, M, S><<<grid_n, kNodeThreads, 0, st>>>(A);
+void launch_update(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
+  launch(k_update<G, L, M, S>, grid_n, kNodeThreads, st, chained, A);
 }
-using UpdateFn = void (*)(int, cudaStream_t, const UpdateArgs&);
+using UpdateFn = void (*)(int, cudaStream_t, bool, const UpdateArgs&);
 const UpdateFn kUpdate[16] = {
     launch_update<0, 0, 0, 0>, launch_update<0, 0, 0, 1>, launch_update<0, 0, 1, 0>, launch_update<0, 0, 1, 1>,
     launch_update<0, 1, 0, 0>, launch_update<0, 1, 0, 1>, launch_update<0, 1, 1, 0>, launch_update<0, 1, 1, 1>,
@@ -1176,30 +1253,30 @@ const UpdateFn kUpdate[16] = {
     launch_update<1, 1, 0, 0>, launch_update<1, 1, 0, 1>, launch_update<1, 1, 1, 0>, launch_update<1, 1, 1, 1>};
 
 template <bool G, bool L, bool S>
-void launch_update_dw(int grid_n, cudaStream_t st, const UpdateArgs& A) {
-  k_update<G, L, false, S, false, false, 0, true><<<grid_n, kNodeThreads, 0, st>>>(A);
+void launch_update_dw(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
+  launch(k_update<G, L, false, S, false, false, 0, true>, grid_n, kNodeThreads, st, chained, A);
 }
 const UpdateFn kUpdateDW[8] = {launch_update_dw<0, 0, 0>, launch_update_dw<0, 0, 1>, launch_update_dw<0, 1, 0>,
                                launch_update_dw<0, 1, 1>, launch_update_dw<1, 0, 0>, launch_update_dw<1, 0, 1>,
                                launch_update_dw<1, 1, 0>, launch_update_dw<1, 1, 1>};
 
 template <bool L, bool S>
-void launch_update_dw_fused(int grid_n, cudaStream_t st, const UpdateArgs& A) {
-  k_update<true, L, false, S, false, true, 0, true><<<grid_n, kNodeThreads, 0, st>>>(A);
+void launch_update_dw_fused(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
+  launch(k_update<true, L, false, S, false, true, 0, true>, grid_n, kNodeThreads, st, chained, A);
 }
 const UpdateFn kUpdateDWFused[4] = {launch_update_dw_fused<0, 0>, launch_update_dw_fused<0, 1>,
                                     launch_update_dw_fused<1, 0>, launch_update_dw_fused<1, 1>};
 
 template <bool L, bool S>
-void launch_update_pair(int grid_n, cudaStream_t st, const UpdateArgs& A) {
-  k_update<true, L, true, S, true><<<grid_n, kNodeThreads, 0, st>>>(A);
+void launch_update_pair(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
+  launch(k_update<true, L, true, S, true>, grid_n, kNodeThreads, st, chained, A);
 }
 const UpdateFn kUpdatePair[4] = {launch_update_pair<0, 0>, launch_update_pair<0, 1>, launch_update_pair<1, 0>,
                                  launch_update_pair<1, 1>};
 
 template <bool L, bool S, bool P, int V = 0>
-void launch_update_fused(int grid_n, cudaStream_t st, const UpdateArgs& A) {
-  k_update<true, L, true, S, P, true, V><<<grid_n, kNodeThreads, 0, st>>>(A);
+void launch_update_fused(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
+  launch(k_update<true, L, true, S, P, true, V>, grid_n, kNodeThreads, st, chained, A);
 }
 // Indexed by variant (0 per-node loop, 1 staged ids, 2 edge-parallel) * 8 +
 // last * 4 + seg * 2 + pair.
@@ -1215,11 +1292,11 @@ const UpdateFn kUpdateFused[24] = {
 
 template <bool M, bool S, bool W = false>
 void launch_step_begin(const DevLevel& D, unsigned long long* key, const DevStatus* st, const SegStop* ss,
-                       cudaStream_t stream) {
-  k_step_begin<M, S, W><<<grid(D.n, kNodeThreads), kNodeThreads, 0, stream>>>(D.n, D.rec, D.rec2, D.rec32, D.old,
-                                                                               D.cbrt_vol, key, st, D.mesh_id, ss);
+                       cudaStream_t stream, bool chained) {
+  launch(k_step_begin<M, S, W>, grid(D.n, kNodeThreads), kNodeThreads, stream, chained, D.n, D.rec, D.rec2, D.rec32,
+         D.old, D.cbrt_vol, key, st, D.mesh_id, ss);
 }
-using StepFn = void (*)(const DevLevel&, unsigned long long*, const DevStatus*, const SegStop*, cudaStream_t);
+using StepFn = void (*)(const DevLevel&, unsigned long long*, const DevStatus*, const SegStop*, cudaStream_t, bool);
 // Indexed by precision (FP64, MIXED, DW) * 2 + seg.
 const StepFn kStepBegin[6] = {launch_step_begin<0, 0>, launch_step_begin<0, 1>, launch_step_begin<1, 0>,
                               launch_step_begin<1, 1>, launch_step_begin<0, 0, 1>, launch_step_begin<0, 1, 1>};
@@ -1235,17 +1312,24 @@ unsigned long long* level_key_used(mgcfd_solver* s, int level) {
 
 template <bool B, bool M, bool S, bool W>
 void launch_prolong(const DevLevel& F, const DevLevel& Cl, const DevStatus* st, const SegStop* ss,
-                    unsigned long long* key, cudaStream_t stream) {
+                    unsigned long long* key, const KeyReset& coarse_keys, cudaStream_t stream, bool chained) {
   const BeginArgs b{F.rec2, F.rec32, F.old, F.cbrt_vol, key};
-  k_prolong<B, M, S, W><<<grid(F.n, kNodeThreads), kNodeThreads, 0, stream>>>(F.n, F.n2mg, F.dvec, F.rec, F.res,
-                                                                               Cl.res, st, F.mesh_id, ss, b);
+  launch(k_prolong<B, M, S, W>, grid(F.n, kNodeThreads), kNodeThreads, stream, chained, F.n, F.n2mg, F.dvec, F.rec,
+         F.res, Cl.res, st, F.mesh_id, ss, b, coarse_keys);
 }
 using ProlongFn = void (*)(const DevLevel&, const DevLevel&, const DevStatus*, const SegStop*, unsigned long long*,
-                           cudaStream_t);
+                           const KeyReset&, cudaStream_t, bool);
 // With the fine level's step begin, indexed by precision (FP64, MIXED, DW) * 2 + seg.
 const ProlongFn kProlongBegin[6] = {launch_prolong<1, 0, 0, 0>, launch_prolong<1, 0, 1, 0>,
                                    launch_prolong<1, 1, 0, 0>, launch_prolong<1, 1, 1, 0>,
                                    launch_prolong<1, 0, 0, 1>, launch_prolong<1, 0, 1, 1>};
+
+KeyReset key_reset(mgcfd_solver* s, int level) {
+  return KeyReset{level_key(s, level), level_key_used(s, level), s->nseg};
+}
+
+// Kernel timing records events between launches, so its launches are plain.
+bool chained(const mgcfd_solver* s) { return !s->opt.time_kernels; }
 
 int precision_index(const mgcfd_solver* s) {
   return s->opt.precision == MGCFD_PRECISION_DW ? 2 : s->opt.precision == MGCFD_PRECISION_MIXED ? 1 : 0;
@@ -1266,20 +1350,15 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
   const bool dw = s->opt.precision == MGCFD_PRECISION_DW;
   const bool timing = s->opt.time_kernels && level == 0;
   const bool seg = s->nseg > 1;
+  const bool pdl = chained(s);
+  const bool transfers = s->L.size() > 1;  // each step's transfer resets its level's keys
   unsigned long long* key = level_key(s, level);
   if (!s->begun) {  // no prolongation began this step: its own begin pass
-    CK(cudaMemsetAsync(key, 0xff, sizeof(unsigned long long) * (size_t)s->nseg, s->stream));
-    kStepBegin[2 * precision_index(s) + (seg ? 1 : 0)](D, key, s->st, seg ? s->seg_stop : nullptr, s->stream);
+    if (!transfers) CK(cudaMemsetAsync(key, 0xff, sizeof(unsigned long long) * (size_t)s->nseg, s->stream));
+    kStepBegin[2 * precision_index(s) + (seg ? 1 : 0)](D, key, s->st, seg ? s->seg_stop : nullptr, s->stream, pdl);
     s->launches++;
   }
   s->begun = false;
-  if (level == 0) {
-    CK(cudaMemsetAsync(&s->st->rms_acc, 0, 2 * sizeof(double), s->stream));  // rms_acc, rho_acc
-    if (seg) {
-      CK(cudaMemsetAsync(s->seg_rms, 0, sizeof(double) * (size_t)s->nseg, s->stream));
-      CK(cudaMemsetAsync(s->seg_rho, 0, sizeof(double) * (size_t)s->nseg, s->stream));
-    }
-  }
   const int et = edge_threads(s);
   const bool pair = mixed && s->opt.accumulation == MGCFD_ACCUM_PAIR32;
   for (int rk = 0; rk < kRK; rk++) {
@@ -1310,14 +1389,11 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
     } else if (D.ne > 0 && !s->fused) {
       const int g = grid(D.ne, et);
       if (dw) {
-        if (s->gather) k_flux_dw<true><<<g, et, 0, s->stream>>>(D.ne, D.e2n, D.w4dw, D.rec2, D.flux, D.fe, s->st);
-        else k_flux_dw<false><<<g, et, 0, s->stream>>>(D.ne, D.e2n, D.w4dw, D.rec2, D.flux, D.fe, s->st);
+        launch(s->gather ? k_flux_dw<true> : k_flux_dw<false>, g, et, s->stream, pdl, D.ne, D.e2n, D.w4dw, D.rec2, D.flux, D.fe, s->st);
       } else if (mixed) {
-        if (s->gather) k_flux_mixed<true><<<g, et, 0, s->stream>>>(D.ne, D.e2n, D.w4f, D.rec32, D.flux, D.fe32, s->st);
-        else k_flux_mixed<false><<<g, et, 0, s->stream>>>(D.ne, D.e2n, D.w4f, D.rec32, D.flux, D.fe32, s->st);
+        launch(s->gather ? k_flux_mixed<true> : k_flux_mixed<false>, g, et, s->stream, pdl, D.ne, D.e2n, D.w4f, D.rec32, D.flux, D.fe32, s->st);
       } else {
-        if (s->gather) k_flux_f64<true><<<g, et, 0, s->stream>>>(D.ne, D.e2n, D.w4, D.rec, D.flux, D.fe, s->st);
-        else k_flux_f64<false><<<g, et, 0, s->stream>>>(D.ne, D.e2n, D.w4, D.rec, D.flux, D.fe, s->st);
+        launch(s->gather ? k_flux_f64<true> : k_flux_f64<false>, g, et, s->stream, pdl, D.ne, D.e2n, D.w4, D.rec, D.flux, D.fe, s->st);
       }
       s->launches++;
       if (time_this) {
@@ -1327,6 +1403,7 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
     }
     UpdateArgs A;
     A.n = D.n; A.level0 = level == 0 && !norms_in_restrict(s); A.inv_div = 1.0 / (double)(kRK + 1 - rk);
+    A.clear_norms = level == 0 && rk == 0 ? s->nseg : 0;
     A.rec = D.rec; A.rec2 = D.rec2; A.rec32 = D.rec32; A.old = D.old; A.flux = D.flux; A.fe = D.fe; A.fe32 = D.fe32;
     A.a_off = D.a_off; A.b_off = D.b_off; A.b_list = D.b_list; A.inv_vol = D.inv_vol; A.bidx = D.bidx;
     A.bdata = D.bdata; A.res = D.res; A.dt_key = key; A.st = s->st;
@@ -1341,7 +1418,7 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
       A.rec2_in = (rk & 1) ? D.rec2b : D.rec2;
       A.rec2 = (rk & 1) ? D.rec2 : D.rec2b;
       A.rec32_in = nullptr;
-      kUpdateDWFused[(last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, A);
+      kUpdateDWFused[(last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, pdl, A);
       if (time_this) {
         CK(cudaEventRecord(ev.second, s->stream));
         s->pending.push_back(ev);
@@ -1352,20 +1429,20 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
       A.rec32_in = (rk & 1) ? D.rec32b : D.rec32;
       A.rec32 = (rk & 1) ? D.rec32 : D.rec32b;
       kUpdateFused[8 * s->fused_variant + ((last ? 4 : 0) | (seg ? 2 : 0) | (pair ? 1 : 0))](grid(D.n, kNodeThreads),
-                                                                                           s->stream, A);
+                                                                                           s->stream, pdl, A);
       if (time_this) {
         CK(cudaEventRecord(ev.second, s->stream));
         s->pending.push_back(ev);
       }
     } else if (mixed && s->gather && pair) {
       A.rec32_in = nullptr;
-      kUpdatePair[(last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, A);
+      kUpdatePair[(last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, pdl, A);
     } else if (dw) {
       A.rec32_in = nullptr;
-      kUpdateDW[(s->gather ? 4 : 0) | (last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, A);
+      kUpdateDW[(s->gather ? 4 : 0) | (last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, pdl, A);
     } else {
       A.rec32_in = nullptr;
-      kUpdate[(s->gather ? 8 : 0) | (last ? 4 : 0) | (mixed ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, A);
+      kUpdate[(s->gather ? 8 : 0) | (last ? 4 : 0) | (mixed ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, pdl, A);
     }
     s->launches++;
     if (s->opt.measure_mem_bound && D.ne > 0) {
@@ -1373,10 +1450,11 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
       s->launches++;
     }
   }
-  // The key this step used, for the step factors a fetch reports (a
-  // prolongation may begin this level's next step before the fetch).
-  CK(cudaMemcpyAsync(level_key_used(s, level), key, sizeof(unsigned long long) * (size_t)s->nseg,
-                     cudaMemcpyDeviceToDevice, s->stream));
+  // The key this step used, for the step factors a fetch reports; the
+  // transfer that follows does this otherwise.
+  if (!transfers)
+    CK(cudaMemcpyAsync(level_key_used(s, level), key, sizeof(unsigned long long) * (size_t)s->nseg,
+                       cudaMemcpyDeviceToDevice, s->stream));
   CK(cudaGetLastError());
   s->steps++;
   return MGCFD_OK;
@@ -1395,12 +1473,10 @@ int enqueue_iteration(mgcfd_solver* s) {
     DevLevel& F = s->L[(size_t)s->level - 1];
     DevLevel& Cl = s->L[(size_t)s->level];
     const SegStop* ss = s->nseg > 1 ? s->seg_stop : nullptr;
-    if (s->level == 1 && norms_in_restrict(s))  // level-0 norms of the step just smoothed
-      k_restrict<true><<<grid(Cl.n, kNodeThreads), kNodeThreads, 0, s->stream>>>(Cl.n, Cl.ch_off, Cl.ch_list, F.rec,
-                                                                                 Cl.rec, F.res, s->st, Cl.mesh_id, ss);
-    else
-      k_restrict<false><<<grid(Cl.n, kNodeThreads), kNodeThreads, 0, s->stream>>>(Cl.n, Cl.ch_off, Cl.ch_list, F.rec,
-                                                                                  Cl.rec, nullptr, s->st, Cl.mesh_id, ss);
+    // With the level-0 norms of the step just smoothed, where the step left them.
+    launch(s->level == 1 && norms_in_restrict(s) ? k_restrict<true> : k_restrict<false>, grid(Cl.n, kNodeThreads),
+           kNodeThreads, s->stream, chained(s), Cl.n, Cl.ch_off, Cl.ch_list, F.rec, Cl.rec, F.res, s->st, Cl.mesh_id,
+           ss, key_reset(s, s->level - 1));
     s->launches++;
     if (s->level == levels - 1) s->up = false;
   } else {
@@ -1408,10 +1484,9 @@ int enqueue_iteration(mgcfd_solver* s) {
     DevLevel& F = s->L[(size_t)s->level];
     DevLevel& Cl = s->L[(size_t)s->level + 1];
     // The fine level's next smoothing step begins in the prolongation.
-    unsigned long long* key = level_key(s, s->level);
-    CK(cudaMemsetAsync(key, 0xff, sizeof(unsigned long long) * (size_t)s->nseg, s->stream));
     kProlongBegin[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](F, Cl, s->st, s->nseg > 1 ? s->seg_stop : nullptr,
-                                                                   key, s->stream);
+                                                                   level_key(s, s->level), key_reset(s, s->level + 1),
+                                                                   s->stream, chained(s));
     s->begun = true;
     s->launches++;
     if (s->level == 0) {
@@ -1421,10 +1496,10 @@ int enqueue_iteration(mgcfd_solver* s) {
   }
   if (s->cycle != cycle0 && s->stop_max_cycles > 0) {  // a V-cycle just ended
     if (s->nseg > 1)
-      k_cycle_end_seg<<<(unsigned)((s->nseg + 127) / 128), 128, 0, s->stream>>>(
-          s->nseg, s->seg_stop, s->seg_rho, s->seg_n0, s->seg_neg, s->seg_bad, s->stop_max_cycles, s->stop_drop);
+      launch(k_cycle_end_seg, grid(s->nseg, 128), 128, s->stream, chained(s), s->nseg, s->seg_stop, s->seg_rho,
+             s->seg_n0, s->seg_neg, s->seg_bad, s->stop_max_cycles, s->stop_drop);
     else
-      k_cycle_end<<<1, 1, 0, s->stream>>>(s->st, (double)s->L[0].n, s->stop_max_cycles, s->stop_drop);
+      launch(k_cycle_end, 1, 1, s->stream, chained(s), s->st, (double)s->L[0].n, s->stop_max_cycles, s->stop_drop);
     s->launches++;
   }
   CK(cudaGetLastError());
@@ -1514,7 +1589,7 @@ int init_state(mgcfd_solver* s) {
   // no prolongation: each of its steps begins on its own.
   s->begun = s->L.size() > 1;
   if (s->begun)
-    kStepBegin[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](s->L[0], level_key(s, 0), s->st, nullptr, s->stream);
+    kStepBegin[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](s->L[0], level_key(s, 0), s->st, nullptr, s->stream, false);
   CK(cudaGetLastError());
   s->cycle = 0; s->level = 0; s->up = true; s->steps = 0; s->launches = 0;
   s->flux_ms = 0.0; s->flux_sweeps = 0; s->status = MGCFD_OK;
