@@ -318,8 +318,9 @@ enum {
   MGCFD_INCREMENT_COLOURED = 4
 };
 enum { MGCFD_RENUMBER_NONE = 0, MGCFD_RENUMBER_SPATIAL = 1, MGCFD_RENUMBER_RCM = 2 };
-/* Node-residual accumulation in mixed precision.  FP64: every FP32 edge flux
- * is widened exactly and added in FP64.  PAIR32: the fluxes enter an
+/* Node-residual accumulation in mixed precision.  FP64: the sum of the FP32
+ * edge fluxes to FP64 accuracy (gather and fused: error-free transformations in
+ * three FP32 words, rounded to FP64 once; atomic: FP64 additions).  PAIR32: the fluxes enter an
  * unevaluated FP32 pair (hi, lo) through error-free TwoSum steps (Knuth,
  * TAOCP vol. 2, 4.2.2) and the pair is added once in FP64 -- within 2^-48 of
  * the exact sum, and no FP64 add per edge. */

@@ -174,10 +174,21 @@ __device__ __forceinline__ NodePrimF store_rec32_from_var(float* rec32, int64_t 
   return q;
 }
 
+__device__ __forceinline__ void unpack_floats(double w, float& lo, float& hi) {
+  uint32_t h, l;
+  unpack_words(w, h, l);
+  lo = __uint_as_float(l);
+  hi = __uint_as_float(h);
+}
+
 __device__ __forceinline__ NodePrimF load_rec32(const float* rec32, int64_t i) {
-  const float4* r = reinterpret_cast<const float4*>(rec32 + 8 * i);
-  const float4 x = r[0], y = r[1];
-  return NodePrimF{x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  const double4_32a r = *reinterpret_cast<const double4_32a*>(rec32 + 8 * i);  // one 32-byte access
+  NodePrimF q;
+  unpack_floats(r.x, q.rho, q.mx);
+  unpack_floats(r.y, q.my, q.mz);
+  unpack_floats(r.z, q.rhoE, q.p);
+  unpack_floats(r.w, q.s, q.rinv);
+  return q;
 }
 
 // The FP32 edge flux, spelled with explicit IEEE intrinsics (never contracted
@@ -762,7 +773,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   // Edge-parallel fused stage: every thread of the block takes part (the
   // barriers are block-wide), whatever its own node's state.
   float ep_hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, ep_lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  double ep_F[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  Sum32 ep_S[5] = {};
   if (FUSED && EP) {
     const int t = threadIdx.x;
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x;
@@ -811,7 +822,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
         for (int v = 0; v < 5; v++) {
           const float x = s_x[5 * (k - c0) + v];
           if (PAIR) two_sum_acc(ep_hi[v], ep_lo[v], x);
-          else ep_F[v] += f2d_bits(x);
+          else sum32_add(ep_S[v], x);
         }
       }
       __syncthreads();
@@ -829,7 +840,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
     double F[5];
     if (FUSED && EP) {
 #pragma unroll
-      for (int k = 0; k < 5; k++) F[k] = PAIR ? f2d_bits(ep_hi[k]) + f2d_bits(ep_lo[k]) : ep_F[k];
+      for (int k = 0; k < 5; k++) F[k] = PAIR ? f2d_bits(ep_hi[k]) + f2d_bits(ep_lo[k]) : sum32_value(ep_S[k]);
     } else if (FUSED && DW) {
       // Node-centric stage in double-word arithmetic: the sum of the fluxes
       // of this node's edges with the node as end a (f(b, a; -h) = -f(a, b; h):
@@ -861,8 +872,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
       // (end a first), summed in k_update's gather order.
       const NodePrimF me = load_rec32(A.rec32_in, i);
       float hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int k = 0; k < 5; k++) F[k] = 0.0;
+      Sum32 sum[5] = {};
       float f[5];
       for (int32_t j = 0; j < er.deg; j++) {
         const bool end_a = j < er.na;
@@ -883,13 +893,11 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
         for (int k = 0; k < 5; k++) {
           const float x = end_a ? f[k] : -f[k];  // node b receives -f
           if (PAIR) two_sum_acc(hi[k], lo[k], x);
-          else F[k] += f2d_bits(x);
+          else sum32_add(sum[k], x);
         }
       }
-      if (PAIR) {
 #pragma unroll
-        for (int k = 0; k < 5; k++) F[k] = f2d_bits(hi[k]) + f2d_bits(lo[k]);
-      }
+      for (int k = 0; k < 5; k++) F[k] = PAIR ? f2d_bits(hi[k]) + f2d_bits(lo[k]) : sum32_value(sum[k]);
     } else if (GATHER && MIXED && PAIR) {
       // Unevaluated FP32 pairs (hi, lo) fed by error-free TwoSum steps;
       // one FP64 add per variable at the end.
@@ -908,6 +916,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
     } else if (GATHER) {
 #pragma unroll
       for (int k = 0; k < 5; k++) F[k] = 0.0;
+      Sum32 sum[5] = {};
       for (int32_t j = 0; j < er.deg; j++) {
         const bool end_a = j < er.na;
         const int64_t e = end_a ? er.a0 + j : A.b_list[end_a ? 0 : er.b0 + j - er.na];
@@ -915,12 +924,16 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
         for (int k = 0; k < 5; k++) {  // F - x as F + (-x): the same bits, one add instruction for both ends
           if (MIXED) {
             const float x = A.fe32[5 * e + k];
-            F[k] += f2d_bits(end_a ? x : -x);
+            sum32_add(sum[k], end_a ? x : -x);
           } else {
             const double x = A.fe[5 * e + k];
             F[k] += end_a ? x : negate(x);
           }
         }
+      }
+      if (MIXED) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) F[k] = sum32_value(sum[k]);
       }
     } else {
       double* fl = A.flux + 5 * i;

@@ -1,5 +1,6 @@
 // Test harness (not part of the library): the FP64 reciprocal, quotient and
-// square root with FP32 seeds of device_math.cuh on host arrays.
+// square root with FP32 seeds and the FP32 sums of device_math.cuh on host
+// arrays.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -16,7 +17,30 @@ __global__ void k_check(int64_t n, const double* __restrict__ a, const double* _
   s[i] = mgcfd::sqrt_fast(b[i]);
 }
 
+// One row of m terms per thread.
+__global__ void k_sum(int64_t n, int m, const float* __restrict__ x, double* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  mgcfd::Sum32 s = {};
+  for (int j = 0; j < m; j++) mgcfd::sum32_add(s, x[i * m + j]);
+  out[i] = mgcfd::sum32_value(s);
+}
+
 }  // namespace
+
+extern "C" int sum_check(int64_t n, int m, const float* x, double* out) {
+  float* d = nullptr;
+  double* o = nullptr;
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&d), sizeof(float) * (size_t)(n * m));
+  if (!e) e = cudaMalloc(reinterpret_cast<void**>(&o), sizeof(double) * (size_t)n);
+  if (!e && !(e = cudaMemcpy(d, x, sizeof(float) * (size_t)(n * m), cudaMemcpyHostToDevice))) {
+    k_sum<<<(unsigned)((n + 127) / 128), 128>>>(n, m, d, o);
+    if (!(e = cudaGetLastError())) e = cudaMemcpy(out, o, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost);
+  }
+  cudaFree(d);
+  cudaFree(o);
+  return (int)e;
+}
 
 // Host buffers in (a, b) and out (1/b, a/b, sqrt(b)); returns a cudaError_t value.
 extern "C" int seed_check(int64_t n, const double* a, const double* b, double* r, double* q, double* s) {

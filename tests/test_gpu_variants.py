@@ -64,19 +64,22 @@ def _seed_inputs(kind):
 
 
 @pytest.fixture(scope="module")
-def seed_check():
+def native():
     here = Path(__file__).resolve().parent
     out = here / "_build" / "libseed_check.so"
     out.parent.mkdir(exist_ok=True)
     subprocess.run([_build._nvcc(), *_build.ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
                     f"-I{_build.CSRC}", str(here / "native" / "seed_check.cu"), "-o", str(out)], check=True,
                    capture_output=True)
-    lib = C.CDLL(str(out))
+    return C.CDLL(str(out))
 
+
+@pytest.fixture(scope="module")
+def seed_check(native):
     def run(a, b):
         outs = [np.empty(len(b)) for _ in range(3)]
         p = [x.ctypes.data_as(C.c_void_p) for x in (a, b, *outs)]
-        assert lib.seed_check(C.c_int64(len(b)), *p) == 0
+        assert native.seed_check(C.c_int64(len(b)), *p) == 0
         return outs
 
     return run
@@ -115,3 +118,42 @@ def test_seeded_forms_keep_the_ieee_special_cases(seed_check):
         ieee = ~nan & ~fast
         assert np.array_equal(got[ieee].view(np.uint64), w[ieee].view(np.uint64))
         assert _ulps(got[fast], ld[fast]).max() <= 0.5 + 2.0 ** -9
+
+
+@pytest.mark.parametrize("terms", [1, 2, 6, 7, 14, 40])
+def test_sum32_is_no_worse_than_fp64_adds(native, terms):
+    """Sum32 over FP32 terms of both signs and of magnitudes 2^40 apart,
+    cancelling ones among them: within half an ulp of the exact sum plus
+    n^2 2^-72 of the terms' magnitudes (and the two roundings of lo + tail and
+    of the value: 2^-53 of a result, 2^-24 * 2^-53 of the magnitudes), which is no
+    more than adding the widened terms one by one in FP64 may lose."""
+    rng = np.random.default_rng(terms)
+    n = 100_000
+    x = np.ldexp(rng.random((n, terms)) * 2 - 1, rng.integers(-20, 21, (n, terms))).astype(np.float32)
+    k = terms // 2
+    x[: n // 2, k:2 * k] = -x[: n // 2, :k] * np.float32(1 + 2.0 ** -20)
+    out = np.empty(n)
+    assert native.sum_check(C.c_int64(n), C.c_int(terms), x.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p)) == 0
+    exact = x.astype(np.longdouble).sum(axis=1)
+    mag = np.abs(x).astype(np.longdouble).sum(axis=1)
+    err = np.abs(out.astype(np.longdouble) - exact)
+    # (long double sums of the references: 64 significand bits or more, 2^-63 of the magnitudes)
+    bound = np.abs(exact) * 2.0 ** -53 + mag * (terms ** 2 * 2.0 ** -72 + 2.0 ** -77 + terms * 2.0 ** -63)
+    assert (err <= bound).all()
+    seq = np.zeros(n)
+    for j in range(terms):
+        seq = seq + x[:, j].astype(np.float64)
+    assert err.sum() <= np.abs(seq.astype(np.longdouble) - exact).sum() * (1 + 1e-9) + float(bound.sum()) * 1e-3
+
+
+def test_sum32_beyond_binary32_and_not_finite(native):
+    f = np.float32
+    x = np.array([[np.inf, 1], [-np.inf, 1], [np.inf, -np.inf], [np.nan, 1], [3e38, 3e38], [-3e38, -3e38], [0.0, -0.0],
+                  [1e-40, 2e-40]], dtype=f)
+    out = np.empty(len(x))
+    assert native.sum_check(C.c_int64(len(x)), C.c_int(2), x.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p)) == 0
+    np.testing.assert_array_equal(out[:2], [np.inf, -np.inf])
+    assert np.isnan(out[2:4]).all()
+    np.testing.assert_array_equal(out[4:6], [np.inf, -np.inf])  # leaves binary32's range
+    assert out[6] == 0.0
+    assert out[7] == float(x[7, 0]) + float(x[7, 1])
