@@ -21,9 +21,9 @@
 //
 // Kernels per smoothing step (euler3d.cpp:467-550):
 //   k_step_begin   nodes  old = var, primitives, dt, block min -> atomicMin
-//                         (a step that a prolongation precedes -- every
-//                         level-0 step after the first -- begins inside
-//                         k_prolong instead, on the state it just wrote)
+//                         (only for a solver's first step and those of a
+//                         one-level solver: the others begin inside the
+//                         transfer before them, on the state it just wrote)
 //   3 x { k_flux   edges  edge flux, +f to a and -f to b (FP64 atomics) or
 //                         f stored per edge (gather strategy)
 //         k_update nodes  gathered flux + boundary flux, time step, flux = 0,
@@ -328,7 +328,7 @@ __device__ __forceinline__ void step_begin_core(int64_t i, bool live, const doub
   }
 }
 
-// The step begin on its own (a step that no prolongation precedes).
+// The step begin on its own (a step that no transfer precedes).
 template <bool MIXED, bool SEG, bool DW = false>
 __global__ void __launch_bounds__(kNodeThreads) k_step_begin(int32_t n, double* rec, double* rec2, float* rec32,
                                                              double* old, const double* __restrict__ cbrt_vol,
@@ -1045,68 +1045,8 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   block_norms(srms, srho, sbad, r2, rr, bad, A.st);
 }
 
-// up_pre/up/up_post (mg.h:29-64) as a gather over each coarse node's children.
-// NORMS (restriction from level 0 of a plain solver): the same pass also
-// takes calc_rms_kernel and count_bad_vals (validation.h:37-44, 102-115) of
-// the level-0 step just finished, since it reads every fine node's state once
-// and the residuals sit beside it.  Its blocks cover about eight fine nodes
-// per thread, so the block reductions are an eighth of those a fine-node
-// kernel would run.
-template <bool NORMS>
-__global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int32_t* __restrict__ ch_off,
-                                                           const int32_t* __restrict__ ch_list, const double* frec,
-                                                           double* crec, const double* fres, DevStatus* st,
-                                                           const int32_t* __restrict__ mesh_id,
-                                                           const SegStop* seg_stop, KeyReset fine_keys) {
-  __shared__ double srms[NORMS ? kNodeThreads : 1], srho[NORMS ? kNodeThreads : 1];
-  __shared__ int sbad[NORMS ? kNodeThreads : 1];
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int32_t lo = c < nc ? ch_off[c] : 0, hi = c < nc ? ch_off[c + 1] : 0;
-  grid_wait();
-  // The same for every thread of the launch, except that the norms' blocks
-  // may set it: one thread reads it for its block, whose reduction synchronises.
-  int halted;
-  if (NORMS) {
-    __shared__ int s_halt;
-    if (threadIdx.x == 0) s_halt = st->halt;
-    __syncthreads();
-    halted = s_halt;
-  } else {
-    halted = st->halt;
-  }
-  reset_keys(fine_keys, halted);
-  if (halted) return;
-  double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sums of squared residuals, one chain per variable
-  int bad = 0;
-  const bool stopped = c < nc && seg_stop && seg_stop[mesh_id[c]].halt;  // a stopped mesh of a batch
-  if (hi > lo && !stopped) {  // no children: state unchanged (avg = 1 on untouched values)
-    double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int32_t j = lo; j < hi; j++) {
-      const int64_t f = ch_list[j];
-      const double4_32a x = *reinterpret_cast<const double4_32a*>(frec + 8 * f);  // one 32-byte access
-      const double r[5] = {x.x, x.y, x.z, x.w, frec[8 * f + 4]};
-#pragma unroll
-      for (int k = 0; k < 5; k++) s[k] += r[k];
-      if (NORMS) {
-        const double* d = fres + 5 * f;
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-          q[k] += d[k] * d[k];
-          bad += not_finite(r[k]) ? 1 : 0;
-        }
-      }
-    }
-    const double avg = 1.0 / (double)(hi - lo);
-    double* r = crec + 8 * c;
-#pragma unroll
-    for (int k = 0; k < 5; k++) r[k] = s[k] * avg;
-  }
-  if (!NORMS) return;
-  block_norms(srms, srho, sbad, ((q[0] + q[1]) + (q[2] + q[3])) + q[4], q[0], bad, st);
-}
-
-// The fine level's step-begin arrays, for a prolongation that begins its
-// next smoothing step.
+// The step-begin arrays of the level that a transfer writes, whose next
+// smoothing step begins in the transfer.
 struct BeginArgs {
   double* rec2;
   float* rec32;
@@ -1115,11 +1055,79 @@ struct BeginArgs {
   unsigned long long* dt_key;
 };
 
-// down_kernel (mg.h:66-88) with the parent offsets precomputed.  BEGIN: the
-// fine level's next smoothing step begins here (step_begin_core on the new
-// state while it is in registers) instead of in a separate pass that reads
-// the level's state again; every thread reaches the block reduction.
-template <bool BEGIN, bool MIXED, bool SEG, bool DW>
+// up_pre/up/up_post (mg.h:29-64) as a gather over each coarse node's children,
+// and the coarse level's step begin on the state just written (as in the
+// prolongation: a launch and a pass over the coarse level fewer; 8^3 mixed
+// V-cycle 95.7 -> 94.2 us, 200^3 2993 -> 2962 us).  Each thread walks its own
+// node's children: staging the block's children rows through shared memory,
+// coalesced, measured slower (200^3 mixed 3108 us), and so did two lanes per
+// coarse node at large sizes (3011 us).
+// NORMS (restriction from level 0 of a plain solver): the same pass also
+// takes calc_rms_kernel and count_bad_vals (validation.h:37-44, 102-115) of
+// the level-0 step just finished, since it reads every fine node's state once
+// and the residuals sit beside it.  Its blocks cover about eight fine nodes
+// per thread, so the block reductions are an eighth of those a fine-node
+// kernel would run.
+template <bool NORMS, bool MIXED, bool SEG, bool DW>
+__global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int32_t* __restrict__ ch_off,
+                                                           const int32_t* __restrict__ ch_list, const double* frec,
+                                                           double* crec, const double* fres, DevStatus* st,
+                                                           const int32_t* __restrict__ mesh_id,
+                                                           const SegStop* seg_stop, BeginArgs B, KeyReset fine_keys) {
+  __shared__ double srms[NORMS ? kNodeThreads : 1], srho[NORMS ? kNodeThreads : 1];
+  __shared__ int sbad[NORMS ? kNodeThreads : 1];
+  __shared__ int s_halt;
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t lo = c < nc ? ch_off[c] : 0, hi = c < nc ? ch_off[c + 1] : 0;
+  grid_wait();
+  if (threadIdx.x == 0) s_halt = st->halt;
+  __syncthreads();
+  const int halted = s_halt;  // block-uniform: the block synchronises below
+  reset_keys(fine_keys, halted);
+  if (halted) return;
+  const bool live = c < nc && !(seg_stop && seg_stop[mesh_id[c]].halt);  // not a stopped mesh of a batch
+  double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sums of squared residuals, one chain per variable
+  int bad = 0;
+  double x[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  if (live) {
+    double* r = crec + 8 * c;
+    if (hi > lo) {
+      for (int32_t j = lo; j < hi; j++) {
+        const int64_t f = ch_list[j];
+        const double4_32a v = *reinterpret_cast<const double4_32a*>(frec + 8 * f);  // one 32-byte access
+        const double u[5] = {v.x, v.y, v.z, v.w, frec[8 * f + 4]};
+#pragma unroll
+        for (int k = 0; k < 5; k++) x[k] += u[k];
+        if (NORMS) {
+          const double* d = fres + 5 * f;
+#pragma unroll
+          for (int k = 0; k < 5; k++) {
+            q[k] += d[k] * d[k];
+            bad += not_finite(u[k]) ? 1 : 0;
+          }
+        }
+      }
+      const double avg = rcp_fast((double)(hi - lo));
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        x[k] *= avg;
+        if (MIXED || DW) r[k] = x[k];  // (FP64: stored with the primitives)
+      }
+    } else {  // no children: state unchanged (avg = 1 on untouched values)
+#pragma unroll
+      for (int k = 0; k < 5; k++) x[k] = r[k];
+    }
+  }
+  step_begin_core<MIXED, SEG, DW>(c, live, x, crec, B.rec2, B.rec32, B.old, B.cbrt_vol, B.dt_key, mesh_id);
+  if (!NORMS) return;
+  block_norms(srms, srho, sbad, ((q[0] + q[1]) + (q[2] + q[3])) + q[4], q[0], bad, st);
+}
+
+// down_kernel (mg.h:66-88) with the parent offsets precomputed.  The fine
+// level's next smoothing step begins here (step_begin_core on the new state
+// while it is in registers) instead of in a separate pass that reads the
+// level's state again; every thread reaches the block reduction.
+template <bool MIXED, bool SEG, bool DW>
 __global__ void __launch_bounds__(kNodeThreads) k_prolong(int32_t nf, const int32_t* __restrict__ n2mg,
                                                           const double4_32a* __restrict__ dvec, double* frec,
                                                           const double* fres, const double* cres, const DevStatus* st,
@@ -1150,11 +1158,13 @@ __global__ void __launch_bounds__(kNodeThreads) k_prolong(int32_t nf, const int3
     v.z -= d.y * (cr[2] - fr[2]);
     v.w -= d.z * (cr[3] - fr[3]);
     v4 -= d.w * (cr[4] - fr[4]);
-    r4[0] = v;
-    frec[8 * i + 4] = v4;
+    if (MIXED || DW) {  // (FP64: stored with the primitives)
+      r4[0] = v;
+      frec[8 * i + 4] = v4;
+    }
     x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; x[4] = v4;
   }
-  if (BEGIN) step_begin_core<MIXED, SEG, DW>(i, live, x, frec, B.rec2, B.rec32, B.old, B.cbrt_vol, B.dt_key, mesh_id);
+  step_begin_core<MIXED, SEG, DW>(i, live, x, frec, B.rec2, B.rec32, B.old, B.cbrt_vol, B.dt_key, mesh_id);
 }
 
 // Far-field terms w.F_ff of every folded boundary row for a new freestream
@@ -1323,19 +1333,32 @@ unsigned long long* level_key_used(mgcfd_solver* s, int level) {
   return s->nseg > 1 ? s->seg_keys + ((size_t)kMaxLevels + level) * s->nseg : &s->st->dt_key_used[level];
 }
 
-template <bool B, bool M, bool S, bool W>
+template <bool M, bool S, bool W>
 void launch_prolong(const DevLevel& F, const DevLevel& Cl, const DevStatus* st, const SegStop* ss,
                     unsigned long long* key, const KeyReset& coarse_keys, cudaStream_t stream, bool chained) {
   const BeginArgs b{F.rec2, F.rec32, F.old, F.cbrt_vol, key};
-  launch(k_prolong<B, M, S, W>, grid(F.n, kNodeThreads), kNodeThreads, stream, chained, F.n, F.n2mg, F.dvec, F.rec,
+  launch(k_prolong<M, S, W>, grid(F.n, kNodeThreads), kNodeThreads, stream, chained, F.n, F.n2mg, F.dvec, F.rec,
          F.res, Cl.res, st, F.mesh_id, ss, b, coarse_keys);
 }
 using ProlongFn = void (*)(const DevLevel&, const DevLevel&, const DevStatus*, const SegStop*, unsigned long long*,
                            const KeyReset&, cudaStream_t, bool);
-// With the fine level's step begin, indexed by precision (FP64, MIXED, DW) * 2 + seg.
-const ProlongFn kProlongBegin[6] = {launch_prolong<1, 0, 0, 0>, launch_prolong<1, 0, 1, 0>,
-                                   launch_prolong<1, 1, 0, 0>, launch_prolong<1, 1, 1, 0>,
-                                   launch_prolong<1, 0, 0, 1>, launch_prolong<1, 0, 1, 1>};
+// Indexed by precision (FP64, MIXED, DW) * 2 + seg.
+const ProlongFn kProlong[6] = {launch_prolong<0, 0, 0>, launch_prolong<0, 1, 0>, launch_prolong<1, 0, 0>,
+                               launch_prolong<1, 1, 0>, launch_prolong<0, 0, 1>, launch_prolong<0, 1, 1>};
+
+template <bool N, bool M, bool S, bool W>
+void launch_restrict(const DevLevel& F, const DevLevel& Cl, DevStatus* st, const SegStop* ss, unsigned long long* key,
+                     const KeyReset& fine_keys, cudaStream_t stream, bool chained) {
+  const BeginArgs b{Cl.rec2, Cl.rec32, Cl.old, Cl.cbrt_vol, key};
+  launch(k_restrict<N, M, S, W>, grid(Cl.n, kNodeThreads), kNodeThreads, stream, chained, Cl.n, Cl.ch_off, Cl.ch_list,
+         F.rec, Cl.rec, F.res, st, Cl.mesh_id, ss, b, fine_keys);
+}
+using RestrictFn = void (*)(const DevLevel&, const DevLevel&, DevStatus*, const SegStop*, unsigned long long*,
+                            const KeyReset&, cudaStream_t, bool);
+const RestrictFn kRestrict[6] = {launch_restrict<0, 0, 0, 0>, launch_restrict<0, 0, 1, 0>, launch_restrict<0, 1, 0, 0>,
+                                 launch_restrict<0, 1, 1, 0>, launch_restrict<0, 0, 0, 1>, launch_restrict<0, 0, 1, 1>};
+// With the level-0 norms: plain solvers with the fused stage, MIXED and DW.
+const RestrictFn kRestrictNorms[2] = {launch_restrict<1, 1, 0, 0>, launch_restrict<1, 0, 0, 1>};
 
 KeyReset key_reset(mgcfd_solver* s, int level) {
   return KeyReset{level_key(s, level), level_key_used(s, level), s->nseg};
@@ -1366,7 +1389,7 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
   const bool pdl = chained(s);
   const bool transfers = s->L.size() > 1;  // each step's transfer resets its level's keys
   unsigned long long* key = level_key(s, level);
-  if (!s->begun) {  // no prolongation began this step: its own begin pass
+  if (!s->begun) {  // no transfer began this step: its own begin pass
     if (!transfers) CK(cudaMemsetAsync(key, 0xff, sizeof(unsigned long long) * (size_t)s->nseg, s->stream));
     kStepBegin[2 * precision_index(s) + (seg ? 1 : 0)](D, key, s->st, seg ? s->seg_stop : nullptr, s->stream, pdl);
     s->launches++;
@@ -1486,10 +1509,13 @@ int enqueue_iteration(mgcfd_solver* s) {
     DevLevel& F = s->L[(size_t)s->level - 1];
     DevLevel& Cl = s->L[(size_t)s->level];
     const SegStop* ss = s->nseg > 1 ? s->seg_stop : nullptr;
-    // With the level-0 norms of the step just smoothed, where the step left them.
-    launch(s->level == 1 && norms_in_restrict(s) ? k_restrict<true> : k_restrict<false>, grid(Cl.n, kNodeThreads),
-           kNodeThreads, s->stream, chained(s), Cl.n, Cl.ch_off, Cl.ch_list, F.rec, Cl.rec, F.res, s->st, Cl.mesh_id,
-           ss, key_reset(s, s->level - 1));
+    // The coarse level's smoothing step begins in the restriction, which also
+    // takes the level-0 norms of the step just smoothed where that left them.
+    const int p = precision_index(s);
+    const RestrictFn fn = s->level == 1 && norms_in_restrict(s) ? kRestrictNorms[p - 1]
+                                                                : kRestrict[2 * p + (s->nseg > 1 ? 1 : 0)];
+    fn(F, Cl, s->st, ss, level_key(s, s->level), key_reset(s, s->level - 1), s->stream, chained(s));
+    s->begun = true;
     s->launches++;
     if (s->level == levels - 1) s->up = false;
   } else {
@@ -1497,7 +1523,7 @@ int enqueue_iteration(mgcfd_solver* s) {
     DevLevel& F = s->L[(size_t)s->level];
     DevLevel& Cl = s->L[(size_t)s->level + 1];
     // The fine level's next smoothing step begins in the prolongation.
-    kProlongBegin[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](F, Cl, s->st, s->nseg > 1 ? s->seg_stop : nullptr,
+    kProlong[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](F, Cl, s->st, s->nseg > 1 ? s->seg_stop : nullptr,
                                                                    level_key(s, s->level), key_reset(s, s->level + 1),
                                                                    s->stream, chained(s));
     s->begun = true;
@@ -1596,10 +1622,10 @@ int init_state(mgcfd_solver* s) {
     if (s->seg_stop) CK(cudaMemsetAsync(s->seg_stop, 0, sizeof(SegStop) * ns, s->stream));
   }
   s->seg_status.assign((size_t)s->nseg, MGCFD_OK);
-  // The first V-cycle's first step begins here; every later V-cycle's
-  // begins in the prolongation that ends the one before, so every V-cycle
-  // (and the captured graph) has the same launches.  A one-level solver has
-  // no prolongation: each of its steps begins on its own.
+  // The first V-cycle's first step begins here; every later step begins in
+  // the transfer before it, so every V-cycle (and the captured graph) has the
+  // same launches.  A one-level solver has no transfers: each of its steps
+  // begins on its own.
   s->begun = s->L.size() > 1;
   if (s->begun)
     kStepBegin[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](s->L[0], level_key(s, 0), s->st, nullptr, s->stream, false);

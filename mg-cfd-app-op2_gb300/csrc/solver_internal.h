@@ -24,7 +24,7 @@ constexpr int kMaxDevices = 64;
 
 struct DevStatus {
   unsigned long long dt_key[kMaxLevels];  // order-preserving key of each level's min_dt (the step
-                                           // begun last: a prolongation begins its fine level's next step)
+                                           // begun last: a transfer begins the next step of the level it writes)
   unsigned long long dt_key_used[kMaxLevels];  // the key each level's last finished step used
   int halt;                                // non-zero: stop all further work
   int neg_dt;                              // min_dt < 0 seen
@@ -124,7 +124,7 @@ struct mgcfd_solver {
   int64_t steps = 0;
   int64_t launches = 0;
   int64_t launches_per_cycle = 0;
-  bool begun = false;   // the next smoothing step's begin is already enqueued (by a prolongation or set-up)
+  bool begun = false;   // the next smoothing step's begin is already enqueued (by a transfer or set-up)
   bool gather = false;  // node-side CSR tables exist (GATHER or FUSED)
   bool fused = false;   // FUSED: flux and update in one node-centric kernel
   bool coloured = false;  // COLOURED: one flux launch per colour class, plain increments
