@@ -190,10 +190,23 @@ __device__ __forceinline__ uint64_t spread3(uint64_t x) {
   return x;
 }
 
+// Marks the nodes that carry boundary entries (groups compute_bnd_node_flux
+// acts on).
+__global__ void k_mark_boundary(int32_t nb, Seg g, const int32_t* __restrict__ b2n, const int32_t* __restrict__ grp,
+                                uint8_t* __restrict__ mark) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nb || grp[k] > 7) return;
+  const int32_t m = seg_of(g.boff, g.nseg, k);
+  const int32_t base = g.noff[m];
+  const int32_t n = b2n[k];
+  if ((uint32_t)n < (uint32_t)(g.noff[m + 1] - base)) mark[base + n] = 1;  // (out of range: reported by k_bnd_keys)
+}
+
 // Same quantisation as spatial_order() in setup.cpp, against the node's own
-// mesh's box.
+// mesh's box.  The marked nodes follow the others (boundary_last).
 __global__ void k_morton(int32_t n, const double* __restrict__ xyz, Seg g, const double* __restrict__ box,
-                         unsigned long long* __restrict__ key, int32_t* __restrict__ val) {
+                         const uint8_t* __restrict__ mark, unsigned long long* __restrict__ key,
+                         int32_t* __restrict__ val) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double* bx = box + 6 * seg_of(g.noff, g.nseg, i);
@@ -204,7 +217,7 @@ __global__ void k_morton(int32_t n, const double* __restrict__ xyz, Seg g, const
     if (t > 2097151.0) t = 2097151.0;
     q[d] = (uint64_t)t;
   }
-  key[i] = (spread3(q[2]) << 2) | (spread3(q[1]) << 1) | spread3(q[0]);
+  key[i] = ((uint64_t)mark[i] << 63) | (spread3(q[2]) << 2) | (spread3(q[1]) << 1) | spread3(q[0]);
   val[i] = (int32_t)i;
 }
 
@@ -605,7 +618,7 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
       k_seg_of<<<nblk(N), T, 0, st>>>(N, g.noff, nseg, nullptr, D.mesh_id);
     }
 
-    // Node order: Morton codes within each mesh, then stably by mesh.
+    // Node order: Morton codes within each mesh, its boundary nodes last, then stably by mesh.
     if (s->opt.renumber == MGCFD_RENUMBER_SPATIAL) {
       unsigned long long *lo, *hi, *key, *key2;
       int32_t *val, *val2;
@@ -616,16 +629,19 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
       CK(cudaMemsetAsync(lo, 0xff, 24 * (size_t)nseg, st));
       CK(cudaMemsetAsync(hi, 0, 24 * (size_t)nseg, st));
       double* box;
-      if ((r = tmp.get(&box, 6 * (size_t)nseg))) return r;
+      uint8_t* mark;
+      if ((r = tmp.get(&box, 6 * (size_t)nseg)) || (r = tmp.get(&mark, (size_t)N))) return r;
+      CK(cudaMemsetAsync(mark, 0, (size_t)N, st));
+      if (NB) k_mark_boundary<<<nblk(NB), T, 0, st>>>(NB, g, I.b2n, I.grp, mark);
       k_bbox<<<nblk(N), T, 0, st>>>(N, I.xyz, g, lo, hi);
       k_box_scale<<<nblk(3 * (int64_t)nseg), T, 0, st>>>(nseg, lo, hi, box);
-      k_morton<<<nblk(N), T, 0, st>>>(N, I.xyz, g, box, key, val);
+      k_morton<<<nblk(N), T, 0, st>>>(N, I.xyz, g, box, mark, key, val);
       if (nseg == 1) {
-        if ((r = sort_pairs(tmp, key, key2, val, D.perm, N, 63, st))) return r;
+        if ((r = sort_pairs(tmp, key, key2, val, D.perm, N, 64, st))) return r;
       } else {
         int32_t *mkey, *mkey2;
         if ((r = tmp.get(&mkey, (size_t)N)) || (r = tmp.get(&mkey2, (size_t)N))) return r;
-        if ((r = sort_pairs(tmp, key, key2, val, val2, N, 63, st))) return r;
+        if ((r = sort_pairs(tmp, key, key2, val, val2, N, 64, st))) return r;
         k_seg_of<<<nblk(N), T, 0, st>>>(N, g.noff, nseg, val2, mkey);
         if ((r = sort_pairs(tmp, mkey, mkey2, val2, D.perm, N, bits_for(nseg - 1), st))) return r;
       }

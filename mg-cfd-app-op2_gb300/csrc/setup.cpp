@@ -73,6 +73,22 @@ void spatial_order(const double* xyz, int32_t n, std::vector<int32_t>* perm) {
   perm->swap(val);
 }
 
+// The solver's node order: the Morton curve with the nodes that carry boundary
+// entries (the groups compute_bnd_node_flux acts on) moved to the end, both
+// parts in curve order.  A warp of a node kernel then holds boundary nodes
+// only or none, except one per mesh; left on the curve, they sat in a fifth
+// of the warps at 100^3 (a third at 48^3), each of which issued their 45 FP64
+// operations for all its lanes.  V-cycle at 48^3: mixed 143.6 -> 127.1 us, FP64
+// 195.7 -> 189.6; 100^3 mixed 550 -> 514; 200^3 FP64 7.07 -> 6.92 ms.  (Listing
+// the boundary nodes of a block in shared memory instead helped 48^3 as much
+// but took L1 from the neighbour gathers: 200^3 mixed 2.94 -> 3.14 ms.)
+void boundary_last(const mgcfd_level_view& v, std::vector<int32_t>* perm) {
+  std::vector<char> isb((size_t)v.nnodes, 0);
+  for (int32_t k = 0; k < v.nbnd; k++)
+    if (v.bnd_group[k] <= 7) isb[(size_t)v.bnd_to_node[k]] = 1;
+  std::stable_partition(perm->begin(), perm->end(), [&](int32_t i) { return !isb[(size_t)i]; });
+}
+
 // Reverse Cuthill-McKee: breadth-first from a low-degree pseudo-peripheral
 // node of each component, neighbours in ascending degree, then reversed.
 void rcm_order(int32_t n, int32_t ne, const int32_t* e2n, std::vector<int32_t>* perm) {
@@ -170,7 +186,7 @@ int prepare_mesh(int32_t nlevels, const mgcfd_level_view* lv, const mgcfd_freest
     P.n = n;
     P.ne = ne;
     // Node order.
-    if (renumber == MGCFD_RENUMBER_SPATIAL) spatial_order(v.coords, n, &P.perm);
+    if (renumber == MGCFD_RENUMBER_SPATIAL) { spatial_order(v.coords, n, &P.perm); boundary_last(v, &P.perm); }
     else if (renumber == MGCFD_RENUMBER_RCM) rcm_order(n, ne, v.edge_to_nodes, &P.perm);
     else { P.perm.resize((size_t)n); for (int32_t i = 0; i < n; i++) P.perm[(size_t)i] = i; }
     P.inv.assign((size_t)n, 0);
