@@ -161,6 +161,9 @@ int64_t estimate_bytes(const std::vector<mgcfd_level_view>& lv, int precision, i
     int64_t node = 8 * 8 + 5 * 8 * 3 + 8 * 3 + 4 * 4 + 32;   // rec, old/res/flux, vol constants, maps, dvec
     int64_t edge = 8 + 32;                                    // e2n, w4
     if (mixed) { node += fused ? 64 : 32; edge += 16; }
+    // (The fused stage's sliced edge lists, up to 2.5 entries of 20 or 36 bytes
+    // per edge, are built when the set-up scratch below, 120 bytes per edge, has
+    // been freed: the peak stays the set-up's.)
     if (dw) {  // rec2, w4dw; fused: rec2b, off2, ent2
       node += 64 + (fused ? 68 : 0);
       edge += 32 + (fused ? 16 : 0);

@@ -13,8 +13,11 @@
 //   fe     [E][5]  f64  per-edge fluxes (gather increment strategy only;
 //                       f32 fe32 in mixed precision)
 //   a_off/b_off/b_list  CSR of each node's edges as end a and as end b
-//                       (gather and fused); b_nbr/b_w4f: the b-side edge data
-//                       in b_list order (fused)
+//                       (gather and fused)
+//   sl_off/sl_nbr/sl_w  fused: each node's edges in slices of 32 nodes, entry j
+//                       of the slice's nodes side by side (see k_slice_fill);
+//                       a level too uneven for that keeps the CSR lists, with
+//                       b_nbr/b_w4f (DW: off2/ent2) beside them
 //   bidx [N] int32 and bdata [NB][12] f64: boundary entries folded per node
 //   n2mg [N], dvec [N] double4: prolongation parent and |dx|,|dy|,|dz|,dist
 //   ch_off/ch_list: restriction children of each coarse node
@@ -56,6 +59,8 @@
 // status word; every later kernel sees it and returns, so the run stops at the
 // same point the reference aborts (with the fused stage, one restriction
 // later).  The host reads the status on synchronize.
+#include <cub/cub.cuh>
+
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -208,6 +213,29 @@ __device__ __forceinline__ void edge_flux_f32(const NodePrimF& a, const NodePrim
   f[3] = __fmaf_rn(fac, __fsub_rn(a.mz, b.mz), __fmaf_rn(pp, w.z, __fmaf_rn(b.mz, uhb, __fmul_rn(a.mz, uha))));
   f[4] = __fmaf_rn(fac, __fsub_rn(a.rhoE, b.rhoE),
                    __fmaf_rn(__fadd_rn(b.rhoE, b.p), uhb, __fmul_rn(__fadd_rn(a.rhoE, a.p), uha)));
+}
+
+// The increment of node `me` from one of its edges, bit for bit the f that
+// edge_flux_f32 gives its end a (me_is_a) or the -f that its end b receives.
+// w: h from me's side (negated at end b).  Every term but one is odd in h or
+// in me - o; the products of the momentum and energy terms are added in the
+// order a, b, the first of them rounded.
+__device__ __forceinline__ void edge_flux_f32_at(const NodePrimF& me, const NodePrimF& o, float4 w, bool me_is_a,
+                                                 float f[5]) {
+  const float mhm = __fmaf_rn(me.mz, w.z, __fmaf_rn(me.my, w.y, __fmul_rn(me.mx, w.x)));
+  const float mho = __fmaf_rn(o.mz, w.z, __fmaf_rn(o.my, w.y, __fmul_rn(o.mx, w.x)));
+  const float uhm = __fmul_rn(mhm, me.rinv), uho = __fmul_rn(mho, o.rinv);
+  const float fac = __fmul_rn(w.w, __fadd_rn(me.s, o.s));
+  const float pp = __fadd_rn(me.p, o.p);
+  const float ua = me_is_a ? uhm : uho, ub = me_is_a ? uho : uhm;
+  auto central = [&](float m, float x) {  // x_a u_a + x_b u_b
+    return __fmaf_rn(me_is_a ? x : m, ub, __fmul_rn(me_is_a ? m : x, ua));
+  };
+  f[0] = __fmaf_rn(fac, __fsub_rn(me.rho, o.rho), __fadd_rn(mhm, mho));
+  f[1] = __fmaf_rn(fac, __fsub_rn(me.mx, o.mx), __fmaf_rn(pp, w.x, central(me.mx, o.mx)));
+  f[2] = __fmaf_rn(fac, __fsub_rn(me.my, o.my), __fmaf_rn(pp, w.y, central(me.my, o.my)));
+  f[3] = __fmaf_rn(fac, __fsub_rn(me.mz, o.mz), __fmaf_rn(pp, w.z, central(me.mz, o.mz)));
+  f[4] = __fmaf_rn(fac, __fsub_rn(me.rhoE, o.rhoE), central(__fadd_rn(me.rhoE, me.p), __fadd_rn(o.rhoE, o.p)));
 }
 
 // 1/vol and cbrt(vol) on the device for both setup paths, so the solver's
@@ -443,6 +471,49 @@ __global__ void k_dw_table_b(int32_t ne, const int2* __restrict__ e2n, const int
   ent2[off2[b] + (a_off[b + 1] - a_off[b]) + (j - b_off[b])] = make_int2(a, (int32_t)((uint32_t)e | 0x80000000u));
 }
 
+// Sliced edge lists of the fused stage.  The nodes of a warp form a slice, as
+// wide as its node with the most edges; entry j of the slice is 32 neighbour
+// ids and 32 weights in lane order (id -1: this node has fewer edges), so a
+// warp reads each round of its edge loop as whole lines.  From the CSR lists
+// each lane read its own node's run: 32 short pieces of as many lines per
+// round, which the L1 pipe paid for (DW at 100^3: 70% of its wavefronts).
+// V-cycle at 100^3, CSR -> sliced: DW 624 -> 584 us, pair sums 472 -> 460, mixed
+// 514 -> 509; at 200^3 3.56 -> 3.47, 2.63 -> 2.57 and 2.90 -> 2.91 ms (there
+// the FP64 node sums' tail, not the lists, holds the mixed stage).  A node's entries keep the gather order,
+// its a-side edges then its b-side ones; the b side has h negated and bit 31 of
+// the id set.
+__global__ void k_slice_width(int32_t n, const int32_t* __restrict__ a_off, const int32_t* __restrict__ b_off,
+                              int32_t* __restrict__ width) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int deg = i < n ? (a_off[i + 1] - a_off[i]) + (b_off[i + 1] - b_off[i]) : 0;
+  const int w = __reduce_max_sync(0xffffffffu, deg);
+  if ((threadIdx.x & 31) == 0 && i < n) width[i >> 5] = w;
+}
+
+__device__ __forceinline__ float4 other_end(float4 w) { return make_float4(-w.x, -w.y, -w.z, w.w); }
+__device__ __forceinline__ double4_32a other_end(double4_32a w) {  // pair words: both words' signs
+  auto neg = [](double p) { return dw_pack(dw_neg(dw_unpack(p))); };
+  return make_double4_32a(neg(w.x), neg(w.y), neg(w.z), w.w);
+}
+
+template <class W>
+__global__ void k_slice_fill(int32_t ne, const int2* __restrict__ e2n, const int32_t* __restrict__ b_list,
+                             const int32_t* __restrict__ a_off, const int32_t* __restrict__ b_off,
+                             const W* __restrict__ w, const int32_t* __restrict__ sl_off, int32_t* __restrict__ nbr,
+                             W* __restrict__ sw) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= ne) return;
+  const int2 ab = e2n[k];
+  int64_t at = ((int64_t)sl_off[ab.x >> 5] + (k - a_off[ab.x])) * 32 + (ab.x & 31);
+  nbr[at] = ab.y;
+  sw[at] = w[k];
+  const int32_t e = b_list[k];
+  const int32_t a = e2n[e].x, b = e2n[e].y;
+  at = ((int64_t)sl_off[b >> 5] + (a_off[b + 1] - a_off[b]) + (k - b_off[b])) * 32 + (b & 31);
+  nbr[at] = (int32_t)((uint32_t)a | 0x80000000u);
+  sw[at] = other_end(w[e]);
+}
+
 // The edge weights as pair words (DW precision), once at set-up, counting
 // the finite non-zero weights outside [2^-70, 2^70): their products with the
 // flow state would leave the pairs' binary32 exponent range.
@@ -562,6 +633,10 @@ struct UpdateArgs {
   const int32_t* off2;     // DW fused: per-node neighbour table
   const int2* ent2;
   const double4_32a* w4dw;
+  const int32_t* sl_off;   // fused: sliced edge lists
+  const int32_t* sl_nbr;
+  const float4* sl_w;
+  const double4_32a* sl_w2;
   float* rec32;
   const double* old;
   double* flux;
@@ -702,6 +777,7 @@ template <bool GATHER, bool LAST, bool MIXED, bool SEG, bool PAIR = false, bool 
 __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED && DW) ? 8 : 0) k_update(UpdateArgs A) {
   constexpr bool STAGE = FV == 1;  // neighbour ids staged by cp.async
   constexpr bool EP = FV == 2;     // edge-parallel ends through shared memory
+  constexpr bool SLICED = FV == 3;  // sliced edge lists
   __shared__ int32_t s_aid[STAGE ? kStageIds : 1], s_bid[STAGE ? kStageIds : 1];
   __shared__ float s_x[EP ? 5 * kEpChunk : 1];
   __shared__ float4 s_me[EP ? 2 * kNodeThreads : 1];
@@ -729,10 +805,16 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   double o[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, Fa[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, ivol = 0.0;
   int32_t bi = -1;
   EdgeRange er{0, 0, 0, 0};
-  int32_t k0 = 0, k1 = 0;  // DW fused: the node's entries
+  int32_t k0 = 0, k1 = 0;  // DW fused: the node's entries; SLICED: the slice's rows
+  int32_t first = -1;      // SLICED: the node's first neighbour
+  const int lane = threadIdx.x & 31;
   if (!GATHER && i < A.n) {  // (the gather forms load them after their edge loop)
     ivol = A.inv_vol[i];
     bi = A.bidx[i];
+  } else if (SLICED && i - lane < A.n) {
+    k0 = A.sl_off[i >> 5];
+    k1 = A.sl_off[(i >> 5) + 1];
+    if (k0 < k1) first = A.sl_nbr[32 * (int64_t)k0 + lane];
   } else if (FUSED && DW && i < A.n) {
     k0 = A.off2[i];
     k1 = A.off2[i + 1];
@@ -852,6 +934,18 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
       const dwf s_me = dw_unpack(A.rec2_in[8 * i + 6]);
       NodeFluxDW acc;
       node_flux_dw_init(acc);
+      if (SLICED) {
+        int32_t next = first;
+        for (int32_t j = k0; j < k1; j++) {
+          const int32_t nb = next;  // the following round's id loads during this edge's arithmetic
+          if (j + 1 < k1) next = A.sl_nbr[32 * ((int64_t)j + 1) + lane];
+          if (nb == -1) continue;
+          const NodePrimDW o = load_prim_dw(A.rec2_in, nb & 0x7fffffff);
+          const double4_32a w = A.sl_w2[32 * (int64_t)j + lane];
+          node_flux_dw_edge(acc, s_me, o, dw_unpack(w.x), dw_unpack(w.y), dw_unpack(w.z), dw_unpack(w.w));
+        }
+        k0 = k1;  // none left for the loop over the node's entries
+      }
       int2 next = k0 < k1 ? A.ent2[k0] : make_int2(0, 0);
       for (int32_t j = k0; j < k1; j++) {
         const int2 en = next;  // the following entry loads during this edge's arithmetic
@@ -871,10 +965,25 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
       // the stage's input primitives exactly as k_flux_mixed computes it
       // (end a first), summed in k_update's gather order.
       const NodePrimF me = load_rec32(A.rec32_in, i);
+      if (SLICED) er.deg = k1 - k0;
+      int32_t next_nb = first;
       float hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
       Sum32 sum[5] = {};
       float f[5];
       for (int32_t j = 0; j < er.deg; j++) {
+        if (SLICED) {
+          const int32_t nb = next_nb;
+          const int64_t row = 32 * ((int64_t)k0 + j) + lane;
+          if (j + 1 < er.deg) next_nb = A.sl_nbr[row + 32];
+          if (nb == -1) continue;
+          edge_flux_f32_at(me, load_rec32(A.rec32_in, nb & 0x7fffffff), A.sl_w[row], nb >= 0, f);
+#pragma unroll
+          for (int k = 0; k < 5; k++) {
+            if (PAIR) two_sum_acc(hi[k], lo[k], f[k]);
+            else sum32_add(sum[k], f[k]);
+          }
+          continue;
+        }
         const bool end_a = j < er.na;
         const int32_t ja = end_a ? er.a0 + j : 0, jb = end_a ? 0 : er.b0 + j - er.na;  // both in range
         int32_t nb;
@@ -1283,12 +1392,15 @@ const UpdateFn kUpdateDW[8] = {launch_update_dw<0, 0, 0>, launch_update_dw<0, 0,
                                launch_update_dw<0, 1, 1>, launch_update_dw<1, 0, 0>, launch_update_dw<1, 0, 1>,
                                launch_update_dw<1, 1, 0>, launch_update_dw<1, 1, 1>};
 
-template <bool L, bool S>
+template <bool L, bool S, int V>
 void launch_update_dw_fused(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
-  launch(k_update<true, L, false, S, false, true, 0, true>, grid_n, kNodeThreads, st, chained, A);
+  launch(k_update<true, L, false, S, false, true, V, true>, grid_n, kNodeThreads, st, chained, A);
 }
-const UpdateFn kUpdateDWFused[4] = {launch_update_dw_fused<0, 0>, launch_update_dw_fused<0, 1>,
-                                    launch_update_dw_fused<1, 0>, launch_update_dw_fused<1, 1>};
+// Indexed by sliced * 4 + last * 2 + seg.
+const UpdateFn kUpdateDWFused[8] = {launch_update_dw_fused<0, 0, 0>, launch_update_dw_fused<0, 1, 0>,
+                                    launch_update_dw_fused<1, 0, 0>, launch_update_dw_fused<1, 1, 0>,
+                                    launch_update_dw_fused<0, 0, 3>, launch_update_dw_fused<0, 1, 3>,
+                                    launch_update_dw_fused<1, 0, 3>, launch_update_dw_fused<1, 1, 3>};
 
 template <bool L, bool S>
 void launch_update_pair(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
@@ -1301,9 +1413,9 @@ template <bool L, bool S, bool P, int V = 0>
 void launch_update_fused(int grid_n, cudaStream_t st, bool chained, const UpdateArgs& A) {
   launch(k_update<true, L, true, S, P, true, V>, grid_n, kNodeThreads, st, chained, A);
 }
-// Indexed by variant (0 per-node loop, 1 staged ids, 2 edge-parallel) * 8 +
-// last * 4 + seg * 2 + pair.
-const UpdateFn kUpdateFused[24] = {
+// Indexed by variant (0 per-node loop over the CSR lists, 1 staged ids, 2
+// edge-parallel, 3 sliced lists) * 8 + last * 4 + seg * 2 + pair.
+const UpdateFn kUpdateFused[32] = {
     launch_update_fused<0, 0, 0, 0>, launch_update_fused<0, 0, 1, 0>, launch_update_fused<0, 1, 0, 0>,
     launch_update_fused<0, 1, 1, 0>, launch_update_fused<1, 0, 0, 0>, launch_update_fused<1, 0, 1, 0>,
     launch_update_fused<1, 1, 0, 0>, launch_update_fused<1, 1, 1, 0>, launch_update_fused<0, 0, 0, 1>,
@@ -1311,7 +1423,10 @@ const UpdateFn kUpdateFused[24] = {
     launch_update_fused<1, 0, 0, 1>, launch_update_fused<1, 0, 1, 1>, launch_update_fused<1, 1, 0, 1>,
     launch_update_fused<1, 1, 1, 1>, launch_update_fused<0, 0, 0, 2>, launch_update_fused<0, 0, 1, 2>,
     launch_update_fused<0, 1, 0, 2>, launch_update_fused<0, 1, 1, 2>, launch_update_fused<1, 0, 0, 2>,
-    launch_update_fused<1, 0, 1, 2>, launch_update_fused<1, 1, 0, 2>, launch_update_fused<1, 1, 1, 2>};
+    launch_update_fused<1, 0, 1, 2>, launch_update_fused<1, 1, 0, 2>, launch_update_fused<1, 1, 1, 2>,
+    launch_update_fused<0, 0, 0, 3>, launch_update_fused<0, 0, 1, 3>, launch_update_fused<0, 1, 0, 3>,
+    launch_update_fused<0, 1, 1, 3>, launch_update_fused<1, 0, 0, 3>, launch_update_fused<1, 0, 1, 3>,
+    launch_update_fused<1, 1, 0, 3>, launch_update_fused<1, 1, 1, 3>};
 
 template <bool M, bool S, bool W = false>
 void launch_step_begin(const DevLevel& D, unsigned long long* key, const DevStatus* st, const SegStop* ss,
@@ -1448,13 +1563,14 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
     A.seg_stop = seg ? s->seg_stop : nullptr;
     A.e2n = D.e2n; A.w4f = D.w4f; A.b_nbr = D.b_nbr; A.b_w4f = D.b_w4f;
     A.rec2_in = nullptr; A.off2 = D.off2; A.ent2 = D.ent2; A.w4dw = D.w4dw;
+    A.sl_off = D.sl_off; A.sl_nbr = D.sl_nbr; A.sl_w = D.sl_w; A.sl_w2 = D.sl_w2;
     if (s->fused && dw) {
       // Stage rk reads the primitives of stage rk and writes those of rk + 1
       // into the other buffer: k_step_begin fills rec2 for stage 0.
       A.rec2_in = (rk & 1) ? D.rec2b : D.rec2;
       A.rec2 = (rk & 1) ? D.rec2 : D.rec2b;
       A.rec32_in = nullptr;
-      kUpdateDWFused[(last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, pdl, A);
+      kUpdateDWFused[(D.sl_nbr ? 4 : 0) | (last ? 2 : 0) | (seg ? 1 : 0)](grid(D.n, kNodeThreads), s->stream, pdl, A);
       if (time_this) {
         CK(cudaEventRecord(ev.second, s->stream));
         s->pending.push_back(ev);
@@ -1464,7 +1580,8 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
       // into the other buffer: k_step_begin fills rec32 for stage 0.
       A.rec32_in = (rk & 1) ? D.rec32b : D.rec32;
       A.rec32 = (rk & 1) ? D.rec32 : D.rec32b;
-      kUpdateFused[8 * s->fused_variant + ((last ? 4 : 0) | (seg ? 2 : 0) | (pair ? 1 : 0))](grid(D.n, kNodeThreads),
+      const int variant = s->fused_variant == 0 && D.sl_nbr ? 3 : s->fused_variant;
+      kUpdateFused[8 * variant + ((last ? 4 : 0) | (seg ? 2 : 0) | (pair ? 1 : 0))](grid(D.n, kNodeThreads),
                                                                                            s->stream, pdl, A);
       if (time_this) {
         CK(cudaEventRecord(ev.second, s->stream));
@@ -1699,32 +1816,88 @@ int colour_edges(mgcfd_solver* s, DevLevel& D) {
   return MGCFD_OK;
 }
 
-// DW precision: one level's primitives as pair words (written by the node
-// kernels) and its edge weights split into pairs, from the FP64 weights.
-// FUSED: also the second primitive buffer and the per-node neighbour table
-// (nb2, w2 from off2), from the CSR tables a_off, b_off and b_list.
-int build_dw_tables(mgcfd_solver* s, DevLevel& D) {
+// The sliced edge lists of every level of a solver with the fused stage
+// (mixed precision without the measured-slower options, and DW), from its CSR
+// tables and weights.  A level whose slices would hold more than 1.25 entries
+// for each edge end -- its neighbouring nodes' edge counts differ much, as on a
+// random graph -- keeps the CSR lists: there the padding costs more than the
+// whole lines save.  (8192 entries are allowed on top, so that small levels,
+// whose last slice is mostly empty, are not ruled out.)
+template <class W>
+int build_slices(mgcfd_solver* s, W* DevLevel::*weights, W* DevLevel::*slice_weights) {
+  const size_t nl = s->L.size();
+  std::vector<int32_t> rows(nl, 0);
+  std::vector<int32_t*> off(nl, nullptr);
+  struct Scratch {
+    cudaStream_t stream;
+    std::vector<void*> p;
+    ~Scratch() { for (void* q : p) cudaFreeAsync(q, stream); }
+  } tmp{s->stream, {}};
   int r;
-  if ((r = s->alloc(&D.rec2, 8 * (size_t)D.n)) || (r = s->alloc(&D.w4dw, (size_t)D.ne))) return r;
-  const int64_t nw = 4 * (int64_t)D.ne;
-  if (nw) {
-    unsigned int* bad = nullptr;
-    unsigned int nbad = 0;
-    CK(cudaMallocAsync(&bad, sizeof(unsigned int), s->stream));
-    CK(cudaMemsetAsync(bad, 0, sizeof(unsigned int), s->stream));
-    k_split_weights<<<grid(nw, 256), 256, 0, s->stream>>>(nw, reinterpret_cast<const double*>(D.w4),
-                                                          reinterpret_cast<double*>(D.w4dw), bad);
-    CK(cudaMemcpyAsync(&nbad, bad, sizeof(unsigned int), cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaFreeAsync(bad, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
-    if (nbad)
-      return set_error(MGCFD_ERR_INVALID, std::to_string(nbad) + " edge weight components outside the DW form's "
-                                          "range [2^-70, 2^70); use FP64 precision for this mesh");
+  for (size_t l = 0; l < nl; l++) {
+    DevLevel& D = s->L[l];
+    if (D.n == 0 || D.ne == 0) continue;
+    const int32_t ns = (D.n + 31) / 32;
+    int32_t* width = nullptr;
+    void* t = nullptr;
+    size_t bytes = 0;
+    if ((r = s->alloc(&D.sl_off, (size_t)ns + 1))) return r;
+    CK(cudaMallocAsync(reinterpret_cast<void**>(&width), sizeof(int32_t) * ((size_t)ns + 1), s->stream));
+    tmp.p.push_back(width);
+    CK(cudaMemsetAsync(width + ns, 0, sizeof(int32_t), s->stream));
+    k_slice_width<<<grid(D.n, 256), 256, 0, s->stream>>>(D.n, D.a_off, D.b_off, width);
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, width, D.sl_off, ns + 1, s->stream));
+    CK(cudaMallocAsync(&t, bytes, s->stream));
+    tmp.p.push_back(t);
+    CK(cub::DeviceScan::ExclusiveSum(t, bytes, width, D.sl_off, ns + 1, s->stream));
+    CK(cudaMemcpyAsync(&rows[l], D.sl_off + ns, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
   }
-  if (s->fused) {
-    if ((r = s->alloc(&D.rec2b, 8 * (size_t)D.n)) || (r = s->alloc(&D.off2, (size_t)D.n + 1)) ||
-        (r = s->alloc(&D.ent2, 2 * (size_t)D.ne)))
+  CK(cudaStreamSynchronize(s->stream));
+  for (size_t l = 0; l < nl; l++) {
+    DevLevel& D = s->L[l];
+    const int64_t entries = 32 * (int64_t)rows[l];
+    if (entries == 0 || rows[l] < 0 || entries > 2 * (int64_t)D.ne + D.ne / 2 + 8192) continue;
+    if ((r = s->alloc(&(D.*slice_weights), (size_t)entries)) || (r = s->alloc(&D.sl_nbr, (size_t)entries))) return r;
+    CK(cudaMemsetAsync(D.sl_nbr, 0xff, sizeof(int32_t) * (size_t)entries, s->stream));
+    k_slice_fill<W><<<grid(D.ne, 256), 256, 0, s->stream>>>(D.ne, D.e2n, D.b_list, D.a_off, D.b_off, D.*weights,
+                                                            D.sl_off, D.sl_nbr, D.*slice_weights);
+  }
+  CK(cudaGetLastError());
+  return MGCFD_OK;
+}
+
+// DW precision: each level's primitives as pair words (written by the node
+// kernels) and its edge weights split into pairs, from the FP64 weights.
+// FUSED: also the second primitive buffer and the sliced edge lists, or, on a
+// level that has none, the per-node neighbour table (ent2 from off2).
+int build_dw_tables(mgcfd_solver* s) {
+  int r;
+  unsigned int* bad = nullptr;
+  unsigned int nbad = 0;
+  CK(cudaMallocAsync(&bad, sizeof(unsigned int), s->stream));
+  CK(cudaMemsetAsync(bad, 0, sizeof(unsigned int), s->stream));
+  for (auto& D : s->L) {
+    if ((r = s->alloc(&D.rec2, 8 * (size_t)D.n)) || (r = s->alloc(&D.w4dw, (size_t)D.ne))) {
+      cudaFreeAsync(bad, s->stream);
       return r;
+    }
+    const int64_t nw = 4 * (int64_t)D.ne;
+    if (nw)
+      k_split_weights<<<grid(nw, 256), 256, 0, s->stream>>>(nw, reinterpret_cast<const double*>(D.w4),
+                                                            reinterpret_cast<double*>(D.w4dw), bad);
+  }
+  CK(cudaMemcpyAsync(&nbad, bad, sizeof(unsigned int), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaFreeAsync(bad, s->stream));
+  CK(cudaStreamSynchronize(s->stream));
+  if (nbad)
+    return set_error(MGCFD_ERR_INVALID, std::to_string(nbad) + " edge weight components outside the DW form's "
+                                        "range [2^-70, 2^70); use FP64 precision for this mesh");
+  if (!s->fused) return MGCFD_OK;
+  if ((r = build_slices(s, &DevLevel::w4dw, &DevLevel::sl_w2))) return r;
+  for (auto& D : s->L) {
+    if ((r = s->alloc(&D.rec2b, 8 * (size_t)D.n))) return r;
+    if (D.sl_nbr) continue;
+    if ((r = s->alloc(&D.off2, (size_t)D.n + 1)) || (r = s->alloc(&D.ent2, 2 * (size_t)D.ne))) return r;
     k_dw_offsets<<<grid((int64_t)D.n + 1, 256), 256, 0, s->stream>>>(D.n, D.a_off, D.b_off, D.off2);
     if (D.ne) {
       k_dw_table_a<<<grid(D.ne, 256), 256, 0, s->stream>>>(D.ne, D.e2n, D.a_off, D.off2, D.ent2);
@@ -1733,6 +1906,28 @@ int build_dw_tables(mgcfd_solver* s, DevLevel& D) {
   }
   CK(cudaGetLastError());
   return MGCFD_OK;
+}
+
+// Mixed precision, FUSED: the second FP32 primitive buffer and the sliced edge
+// lists, or, on a level that has none, the b-side copies in b_list order.
+int build_fused_tables(mgcfd_solver* s) {
+  int r;
+  if (s->fused_variant == 0 && (r = build_slices(s, &DevLevel::w4f, &DevLevel::sl_w))) return r;
+  for (auto& D : s->L) {
+    if ((r = s->alloc(&D.rec32b, 8 * (size_t)D.n))) return r;
+    if (D.sl_nbr) continue;
+    if ((r = s->alloc(&D.b_nbr, (size_t)D.ne)) || (r = s->alloc(&D.b_w4f, (size_t)D.ne))) return r;
+    if (D.ne > 0)
+      k_bside<<<grid(D.ne, 256), 256, 0, s->stream>>>(D.ne, D.b_list, D.e2n, D.w4f, D.b_nbr, D.b_w4f);
+  }
+  CK(cudaGetLastError());
+  return MGCFD_OK;
+}
+
+// The tables of the solver's own form, once every level's are in place.
+int build_form_tables(mgcfd_solver* s) {
+  if (s->opt.precision == MGCFD_PRECISION_DW) return build_dw_tables(s);
+  return s->fused ? build_fused_tables(s) : MGCFD_OK;
 }
 
 // Increment strategy: AUTO is FP64 atomics for FP64, and the fused
@@ -1843,10 +2038,7 @@ extern "C" int mgcfd_solver_create(int32_t nlevels, const mgcfd_level_view* leve
           (r = s->upload(&D.b_off, p.b_off.data(), (size_t)p.n + 1)) ||
           (r = s->upload(&D.b_list, p.b_list.data(), (size_t)p.ne)))
         return r;
-      if (s->fused) r = build_fused_tables(s.get(), D);
-      else if (mixed) r = s->alloc(&D.fe32, 5 * (size_t)p.ne);
-      else r = s->alloc(&D.fe, 5 * (size_t)p.ne);
-      if (r) return r;
+      if (!s->fused && (r = mixed ? s->alloc(&D.fe32, 5 * (size_t)p.ne) : s->alloc(&D.fe, 5 * (size_t)p.ne))) return r;
     } else {
       if ((r = s->alloc(&D.flux, 5 * (size_t)p.n))) return r;
     }
@@ -1860,10 +2052,9 @@ extern "C" int mgcfd_solver_create(int32_t nlevels, const mgcfd_level_view* leve
     // The host vectors of this level die at the end of create: finish the copies first.
     CK(cudaStreamSynchronize(s->stream));
   }
-  for (auto& D : s->L) {
+  for (auto& D : s->L)
     if (s->coloured && (r = colour_edges(s.get(), D))) return r;
-    if (s->opt.precision == MGCFD_PRECISION_DW && (r = build_dw_tables(s.get(), D))) return r;
-  }
+  if ((r = build_form_tables(s.get()))) return r;
   if ((r = s->alloc(&s->st, 1)) || (r = s->alloc(&s->fetch_buf, 5 * max_n))) return r;
   if ((r = init_state(s.get()))) return r;
   CK(cudaStreamSynchronize(s->stream));
@@ -1916,8 +2107,7 @@ extern "C" int mgcfd_batch_create(int32_t nmeshes, int32_t nlevels, const mgcfd_
   s->nseg = nmeshes;
   s->L.resize((size_t)nlevels);
   if ((r = device_prepare(s.get(), meshes))) return r;
-  for (auto& D : s->L)
-    if (s->opt.precision == MGCFD_PRECISION_DW && (r = build_dw_tables(s.get(), D))) return r;
+  if ((r = build_form_tables(s.get()))) return r;
   size_t max_n = 0;
   for (auto& D : s->L) max_n = std::max(max_n, (size_t)D.n);
   const size_t ns = (size_t)nmeshes;
@@ -1971,18 +2161,6 @@ extern "C" int mgcfd_solver_run(mgcfd_solver* s, int32_t ncycles) {
       if (r) return r;
     }
   }
-  return MGCFD_OK;
-}
-
-int mgcfd::build_fused_tables(mgcfd_solver* s, DevLevel& D) {
-  if (s->opt.precision == MGCFD_PRECISION_DW) return MGCFD_OK;  // its own tables: build_dw_tables
-  int r;
-  if ((r = s->alloc(&D.rec32b, 8 * (size_t)D.n)) || (r = s->alloc(&D.b_nbr, (size_t)D.ne)) ||
-      (r = s->alloc(&D.b_w4f, (size_t)D.ne)))
-    return r;
-  if (D.ne > 0)
-    k_bside<<<(unsigned)((D.ne + 255) / 256), 256, 0, s->stream>>>(D.ne, D.b_list, D.e2n, D.w4f, D.b_nbr, D.b_w4f);
-  CK(cudaGetLastError());
   return MGCFD_OK;
 }
 

@@ -72,6 +72,12 @@ struct DevLevel {
   double* rec2 = nullptr;         // DW: [N][8] node primitives as pair words (dw_math.cuh)
   double4_32a* w4dw = nullptr;    // DW: [E] w4 as pair words
   double* rec2b = nullptr;        // DW fused: second primitive buffer (stages ping-pong)
+  // Fused: sliced edge lists (k_slice_fill): sl_off [slices + 1] rows of 32 entries, then per entry the
+  // neighbour (bit 31: end b, -1: none) and the weights (mixed: sl_w, DW: sl_w2); null: CSR lists instead.
+  int32_t* sl_off = nullptr;
+  int32_t* sl_nbr = nullptr;
+  float4* sl_w = nullptr;
+  double4_32a* sl_w2 = nullptr;
   int32_t* off2 = nullptr;        // DW fused: [N+1] each node's entries in ent2 (a_off + b_off)
   int2* ent2 = nullptr;           // DW fused: [2E] a node's a-side edges, then its b-side ones: (neighbour,
                                   // edge index, bit 31 set on the b side)
@@ -173,10 +179,6 @@ struct MeshInput {
 // meshes (concatenated per level, each renumbered on its own), device_setup.cu.
 // For one mesh the results equal prepare_mesh() in setup.cpp.
 int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes);
-
-// FUSED increment: the second FP32 primitive buffer and the b-side copies
-// (b_nbr, b_w4f) of a level whose e2n, w4f and b_list are in place.
-int build_fused_tables(mgcfd_solver* s, DevLevel& D);
 
 // Re-initialises a plain solver for a new freestream (Mach, angle of
 // attack): far-field boundary terms, state and counters, as a fresh solver
