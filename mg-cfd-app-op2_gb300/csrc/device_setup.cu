@@ -445,6 +445,15 @@ __global__ void k_nonempty(int32_t nn, const int32_t* __restrict__ off, int32_t*
   if (i < nn) flag[i] = off[i + 1] > off[i] ? 1 : 0;
 }
 
+// Rows of each slice of 32 nodes: its node with the most edges.
+__global__ void k_slice_width(int32_t n, const int32_t* __restrict__ a_off, const int32_t* __restrict__ b_off,
+                              int32_t* __restrict__ width) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int deg = i < n ? (a_off[i + 1] - a_off[i]) + (b_off[i + 1] - b_off[i]) : 0;
+  const int w = __reduce_max_sync(0xffffffffu, deg);
+  if ((threadIdx.x & 31) == 0 && i < n) width[i >> 5] = w;
+}
+
 // ---- multigrid ----------------------------------------------------------------
 
 // Fine node f (new global id) of mesh m: its coarse node (new global id),
@@ -549,14 +558,14 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
   for (int m = 0; m < nseg; m++) ffs[(size_t)m] = meshes[(size_t)m].ff;
   int32_t* dmeta;
   mgcfd_freestream* dff;
-  unsigned* fin;  // fin[0]: out-of-range map entries; fin[1 + l]: folded boundary rows of level l
+  unsigned* fin;  // fin[0]: out-of-range map entries; fin[1 + l]: folded boundary rows of level l, then slice rows
   if ((r = tmp.get(&dmeta, meta.size())) || (r = tmp.get(&dff, (size_t)nseg)) ||
-      (r = tmp.get(&fin, 1 + (size_t)nlevels)))
+      (r = tmp.get(&fin, 1 + 2 * (size_t)nlevels)))
     return r;
   unsigned* err = fin;
   CK(cudaMemcpyAsync(dmeta, meta.data(), 4 * meta.size(), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(dff, ffs.data(), sizeof(mgcfd_freestream) * (size_t)nseg, cudaMemcpyHostToDevice, st));
-  CK(cudaMemsetAsync(fin, 0, sizeof(unsigned) * (1 + (size_t)nlevels), st));
+  CK(cudaMemsetAsync(fin, 0, sizeof(unsigned) * (1 + 2 * (size_t)nlevels), st));
   auto seg = [&](int l) {
     const int32_t* M = dmeta + per * (size_t)l;
     return Seg{nseg, M, M + (nseg + 1), M + 2 * (nseg + 1), M + 3 * (nseg + 1), dff};
@@ -610,7 +619,8 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
     double* w4all = nullptr;
     if (mixed) { if ((r = tmp.get(&w4all, 4 * (size_t)NE))) return r; }
     else { if ((r = s->alloc(&D.w4, (size_t)NE))) return r; w4all = reinterpret_cast<double*>(D.w4); }
-    if (s->gather && ((r = s->alloc(&D.a_off, (size_t)N + 1)) || (r = s->alloc(&D.b_off, (size_t)N + 1)) ||
+    const bool lists = wants_edge_lists(s, N);
+    if (lists && ((r = s->alloc(&D.a_off, (size_t)N + 1)) || (r = s->alloc(&D.b_off, (size_t)N + 1)) ||
                       (r = s->alloc(&D.b_list, (size_t)NE))))
       return r;
     if (nseg > 1) {
@@ -688,7 +698,7 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
         if (mixed) k_edge_finalize<true><<<nblk(NE), T, 0, st>>>(NE, g, key2, order, wd, flip, D.e2n, w4all, acnt, bcnt);
         else k_edge_finalize<false><<<nblk(NE), T, 0, st>>>(NE, g, key2, order, wd, flip, D.e2n, w4all, acnt, bcnt);
       }
-      if (s->gather) {
+      if (lists) {
         int32_t *bkey, *bval, *bkey2;
         if ((r = tmp.get(&bkey, (size_t)NE)) || (r = tmp.get(&bval, (size_t)NE)) || (r = tmp.get(&bkey2, (size_t)NE)))
           return r;
@@ -696,6 +706,14 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
         if (NE) {
           k_b_pairs<<<nblk(NE), T, 0, st>>>(NE, D.e2n, bkey, bval);
           if ((r = sort_pairs(tmp, bkey, bkey2, bval, D.b_list, NE, bits_for(N), st))) return r;
+        }
+        if (wants_slices(s, N)) {
+          const int32_t ns = (N + 31) / 32;
+          int32_t* width;
+          if ((r = tmp.get(&width, (size_t)ns + 1)) || (r = s->alloc(&D.sl_off, (size_t)ns + 1))) return r;
+          k_slice_width<<<nblk(N), T, 0, st>>>(N, D.a_off, D.b_off, width);
+          if ((r = offsets(tmp, width, D.sl_off, ns, st))) return r;
+          k_copy1<<<1, 1, 0, st>>>(D.sl_off + ns, fin + 1 + nlevels + l);
         }
       }
     }
@@ -763,10 +781,13 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
     if ((r = offsets(tmp, cnt, Cl.ch_off, NC, st))) return r;
   }
   CK(cudaGetLastError());
-  std::vector<unsigned> h_fin(1 + (size_t)nlevels, 0);
+  std::vector<unsigned> h_fin(1 + 2 * (size_t)nlevels, 0);
   CK(cudaMemcpyAsync(h_fin.data(), fin, sizeof(unsigned) * h_fin.size(), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  for (int l = 0; l < nlevels; l++) s->L[(size_t)l].nbrows = (int32_t)h_fin[1 + (size_t)l];
+  for (int l = 0; l < nlevels; l++) {
+    s->L[(size_t)l].nbrows = (int32_t)h_fin[1 + (size_t)l];
+    s->L[(size_t)l].sl_rows = (int32_t)h_fin[1 + (size_t)(nlevels + l)];
+  }
   if (h_fin[0])
     return set_error(MGCFD_ERR_INVALID, "mesh has " + std::to_string(h_fin[0]) + " map entries out of range");
   return MGCFD_OK;

@@ -59,13 +59,12 @@
 // status word; every later kernel sees it and returns, so the run stops at the
 // same point the reference aborts (with the fused stage, one restriction
 // later).  The host reads the status on synchronize.
-#include <cub/cub.cuh>
-
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <type_traits>
 #include <mutex>
 #include <vector>
 
@@ -482,21 +481,15 @@ __global__ void k_dw_table_b(int32_t ne, const int2* __restrict__ e2n, const int
 // the FP64 node sums' tail, not the lists, holds the mixed stage).  A node's entries keep the gather order,
 // its a-side edges then its b-side ones; the b side has h negated and bit 31 of
 // the id set.
-__global__ void k_slice_width(int32_t n, const int32_t* __restrict__ a_off, const int32_t* __restrict__ b_off,
-                              int32_t* __restrict__ width) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int deg = i < n ? (a_off[i + 1] - a_off[i]) + (b_off[i + 1] - b_off[i]) : 0;
-  const int w = __reduce_max_sync(0xffffffffu, deg);
-  if ((threadIdx.x & 31) == 0 && i < n) width[i >> 5] = w;
-}
-
+template <bool DW>
 __device__ __forceinline__ float4 other_end(float4 w) { return make_float4(-w.x, -w.y, -w.z, w.w); }
-__device__ __forceinline__ double4_32a other_end(double4_32a w) {  // pair words: both words' signs
-  auto neg = [](double p) { return dw_pack(dw_neg(dw_unpack(p))); };
+template <bool DW>
+__device__ __forceinline__ double4_32a other_end(double4_32a w) {  // DW: pair words, both words' signs
+  auto neg = [](double p) { return DW ? dw_pack(dw_neg(dw_unpack(p))) : -p; };
   return make_double4_32a(neg(w.x), neg(w.y), neg(w.z), w.w);
 }
 
-template <class W>
+template <class W, bool DW>
 __global__ void k_slice_fill(int32_t ne, const int2* __restrict__ e2n, const int32_t* __restrict__ b_list,
                              const int32_t* __restrict__ a_off, const int32_t* __restrict__ b_off,
                              const W* __restrict__ w, const int32_t* __restrict__ sl_off, int32_t* __restrict__ nbr,
@@ -511,7 +504,7 @@ __global__ void k_slice_fill(int32_t ne, const int2* __restrict__ e2n, const int
   const int32_t a = e2n[e].x, b = e2n[e].y;
   at = ((int64_t)sl_off[b >> 5] + (a_off[b + 1] - a_off[b]) + (k - b_off[b])) * 32 + (b & 31);
   nbr[at] = (int32_t)((uint32_t)a | 0x80000000u);
-  sw[at] = other_end(w[e]);
+  sw[at] = other_end<DW>(w[e]);
 }
 
 // The edge weights as pair words (DW precision), once at set-up, counting
@@ -628,6 +621,8 @@ struct UpdateArgs {
   int32_t clear_norms;  // first stage at level 0: the number of norm accumulators to clear, else 0
   double inv_div;       // 1 / (RK + 1 - rk)
   double* rec;
+  const double* rec_in;    // FP64, k_stage_small: the stage's input records
+  double* rec_out;         // ... and the next stage's
   double* rec2;            // DW: the next stage's primitives as pairs
   const double* rec2_in;   // DW fused: the stage's input primitives
   const int32_t* off2;     // DW fused: per-node neighbour table
@@ -1154,6 +1149,223 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   block_norms(srms, srho, sbad, r2, rr, bad, A.st);
 }
 
+// One RK stage of a small level, eight threads per node (plain solvers).
+// A small level's stage is latency: k_update with the fused stage walks a
+// node's edges one gather after the other, and the FP64 form takes a flux
+// launch and an update launch per stage.  Here each of a node's eight lanes
+// loads one of its edges' ends (ids and weights before the wait) and computes
+// that edge's terms; through shared memory lane v then sums variable v over
+// the edges in list order and updates it, and all lanes take the primitives.
+// For MIXED and DW the sums see the operands of k_update's in the same order:
+// the same bits, so a level gives one result whichever kernel ran it (a batch
+// runs k_update).  FP64 replaces the atomics by sums in a fixed order and the
+// edge's flux is computed at both ends.
+// P: 0 FP64, 1 MIXED, 2 DW.
+constexpr int kSmallLanes = 8;
+constexpr int kSmallNodes = kNodeThreads / kSmallLanes;  // nodes per block: half a slice
+
+struct DwTerm {  // one product (or value) of a double-word sum, as acc_add_prod adds it
+  float p, e;
+};
+
+__device__ __forceinline__ DwTerm dw_term(dwf x, dwf y) {
+  const dwacc t = acc_prod(x, y);
+  return DwTerm{t.s, t.c};
+}
+
+__device__ __forceinline__ void acc_add_term(dwacc& a, DwTerm t) {
+  float s, q;
+  two_sum(a.s, t.p, s, q);
+  a.s = s;
+  a.c = __fadd_rn(a.c, __fadd_rn(q, t.e));
+}
+
+__device__ __forceinline__ dwf shfl_dw(dwf x, int lane) {
+  return dwf{__shfl_sync(0xffffffffu, x.h, lane, kSmallLanes), __shfl_sync(0xffffffffu, x.l, lane, kSmallLanes)};
+}
+
+template <int P, bool LAST, bool PAIR>
+__global__ void __launch_bounds__(kNodeThreads) k_stage_small(UpdateArgs A) {
+  constexpr bool FP64 = P == 0, MIXED = P == 1, DW = P == 2;
+  constexpr int kTerms = DW ? 26 : 5;  // words per edge end
+  using Word = std::conditional_t<FP64, double, float>;
+  __shared__ Word s_f[kSmallNodes][kSmallLanes][kTerms + (kTerms % 2 == 0)];
+  __shared__ double srms[LAST ? kNodeThreads : 1], srho[LAST ? kNodeThreads : 1];
+  __shared__ int sbad[LAST ? kNodeThreads : 1];
+  __shared__ int s_halt;
+  const int u = threadIdx.x / kSmallLanes, l = threadIdx.x % kSmallLanes;
+  const int64_t i = (int64_t)blockIdx.x * kSmallNodes + u;
+  const bool in = i < A.n;
+  // Constant tables before the wait: the slice's width is the block's.
+  const int64_t i0 = (int64_t)blockIdx.x * kSmallNodes;
+  const int32_t k0 = A.sl_off[i0 >> 5], rows = A.sl_off[(i0 >> 5) + 1] - k0;
+  int32_t nb = -1;
+  float4 w{};
+  double4_32a w2{};
+  auto load_entry = [&](int32_t j) {
+    nb = -1;
+    if (!in || j >= rows) return;
+    const int64_t at = 32 * ((int64_t)k0 + j) + (i & 31);
+    nb = A.sl_nbr[at];
+    if (MIXED) w = A.sl_w[at];
+    else w2 = A.sl_w2[at];
+  };
+  load_entry(l);
+  const double ivol = in ? A.inv_vol[i] : 0.0;
+  const int32_t bi = in ? A.bidx[i] : -1;
+  grid_wait();
+  if (threadIdx.x == 0) s_halt = A.st->halt;
+  if (A.clear_norms && blockIdx.x == 0 && threadIdx.x == 0) {  // this step's norms start from zero
+    A.st->rms_acc = 0.0;
+    A.st->rho_acc = 0.0;
+  }
+  const double min_dt = dkey_inv(*A.dt_key);
+  NodePrim me{}, o{};
+  NodePrimF mef{}, of{};
+  NodePrimDW med{}, od{};
+  auto load_other = [&] {
+    if (nb == -1) return;
+    const int32_t id = nb & 0x7fffffff;
+    if (FP64) o = load_rec(A.rec_in, id);
+    if (MIXED) of = load_rec32(A.rec32_in, id);
+    if (DW) od = load_prim_dw(A.rec2_in, id);
+  };
+  load_other();
+  double old = 0.0;
+  if (in) {
+    if (FP64) me = load_rec(A.rec_in, i);
+    if (MIXED) mef = load_rec32(A.rec32_in, i);
+    if (DW) med = load_prim_dw(A.rec2_in, i);
+    if (l < 5) old = A.old[5 * i + l];
+  }
+  __syncthreads();
+  if (s_halt) return;  // block-uniform: the reduction below synchronises
+  if (min_dt < 0.0) {  // euler3d.cpp:480: abort before the step factor is used
+    if (threadIdx.x == 0) { A.st->neg_dt = 1; atomicOr(&A.st->halt, 1); }
+    return;
+  }
+  // The edges, eight at a time; lane v < 5 sums variable v.
+  double F = 0.0;
+  float hi = 0.0f, lo = 0.0f;
+  Sum32 sum = {};
+  dwacc S{0.0f, 0.0f}, X{0.0f, 0.0f};  // DW: increment v; H_v (v = 1..3), FAC (v = 0)
+  for (int32_t j0 = 0; j0 < rows; j0 += kSmallLanes) {
+    if (j0 > 0) {
+      load_entry(j0 + l);
+      load_other();
+      __syncwarp();
+    }
+    Word* out = s_f[u][l];
+    if (nb == -1) {
+#pragma unroll
+      for (int k = 0; k < kTerms; k++) out[k] = (Word)0;
+    } else if constexpr (FP64) {
+      double f[5];
+      edge_flux(me, o, w2.x, w2.y, w2.z, w2.w, f);
+#pragma unroll
+      for (int k = 0; k < 5; k++) out[k] = f[k];
+    } else if constexpr (MIXED) {
+      float f[5];
+      edge_flux_f32_at(mef, of, w, nb >= 0, f);
+#pragma unroll
+      for (int k = 0; k < 5; k++) out[k] = f[k];
+    } else {  // node_flux_dw_edge's products
+      const dwf hx = dw_unpack(w2.x), hy = dw_unpack(w2.y), hz = dw_unpack(w2.z);
+      const dwf fac = dw_mul(dw_unpack(w2.w), dw_add(med.s, od.s));
+      dwacc t = acc_prod(od.mx, hx);
+      acc_add_prod(t, od.my, hy);
+      acc_add_prod(t, od.mz, hz);
+      const dwf uhb = dw_mul(acc_dw(t), od.rinv);
+      const dwf gb = dw_add(uhb, dw_neg(fac));
+      const DwTerm q[13] = {dw_term(od.rho, gb),  DwTerm{fac.h, fac.l}, dw_term(od.mx, gb), dw_term(od.p, hx),
+                            DwTerm{hx.h, hx.l},   dw_term(od.my, gb),   dw_term(od.p, hy),  DwTerm{hy.h, hy.l},
+                            dw_term(od.mz, gb),   dw_term(od.p, hz),    DwTerm{hz.h, hz.l}, dw_term(od.rhoE, gb),
+                            dw_term(od.p, uhb)};
+#pragma unroll
+      for (int k = 0; k < 13; k++) { out[2 * k] = q[k].p; out[2 * k + 1] = q[k].e; }
+    }
+    __syncwarp();
+    const int m = rows - j0 < kSmallLanes ? rows - j0 : kSmallLanes;
+    if (l < 5) {
+      for (int e = 0; e < m; e++) {
+        const Word* x = s_f[u][e];
+        if constexpr (FP64) {
+          F += x[l];
+        } else if constexpr (MIXED) {
+          if (PAIR) two_sum_acc(hi, lo, x[l]);
+          else sum32_add(sum, x[l]);
+        } else {
+          const int at = l == 0 ? 0 : 6 * l - 2;  // this lane's terms: 0..1, 2..4, 5..7, 8..10, 11..12
+          auto term = [&](int k) { return DwTerm{x[at + 2 * k], x[at + 2 * k + 1]}; };
+          acc_add_term(S, term(0));
+          if (l > 0) acc_add_term(S, term(1));
+          if (l < 4) acc_add_term(X, term(l == 0 ? 1 : 2));
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if constexpr (MIXED) F = PAIR ? f2d_bits(hi) + f2d_bits(lo) : sum32_value(sum);
+  if constexpr (DW) {  // node_flux_dw_finish
+    const dwf own = acc_dw(X);
+    const dwf fac = shfl_dw(own, 0), hx = shfl_dw(own, 1), hy = shfl_dw(own, 2), hz = shfl_dw(own, 3);
+    dwacc t = acc_prod(med.mx, hx);
+    acc_add_prod(t, med.my, hy);
+    acc_add_prod(t, med.mz, hz);
+    const dwf uh = dw_mul(acc_dw(t), med.rinv);
+    const dwf g = dw_add(uh, fac);
+    acc_add_prod(S, l == 0 ? med.rho : l == 1 ? med.mx : l == 2 ? med.my : l == 3 ? med.mz : med.rhoE, g);
+    if (l > 0) acc_add_prod(S, med.p, l == 1 ? hx : l == 2 ? hy : l == 3 ? hz : uh);
+    F = acc_to_double(S);
+  }
+  if (__any_sync(0xffffffffu, bi >= 0)) {
+    double G[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) G[k] = __shfl_sync(0xffffffffu, F, k, kSmallLanes);
+    if (bi >= 0) {
+      if (!FP64) {
+        const double4_32a* r = reinterpret_cast<const double4_32a*>(A.rec + 8 * i);
+        const double4_32a x = r[0];
+        me = node_prim(x.x, x.y, x.z, x.w, r[1].x);
+      }
+      add_boundary(me, A.bdata + 12 * (int64_t)bi, G);
+      F = l == 0 ? G[0] : l == 1 ? G[1] : l == 2 ? G[2] : l == 3 ? G[3] : G[4];
+    }
+  }
+  const double factor = (min_dt * ivol) * A.inv_div;  // step_factor / (RK+1-rk)
+  const double v = old + factor * F;
+  double x[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) x[k] = __shfl_sync(0xffffffffu, v, k, kSmallLanes);
+  grid_trigger();
+  double r2 = 0.0, rr = 0.0;
+  int bad = 0;
+  if (in && l < 5 && (LAST || (!FP64 && bi >= 0))) A.rec[8 * i + l] = v;  // (k_update: which stages store the state)
+  if (LAST) {
+    if (in && l < 5) {
+      const double d = v - old;
+      A.res[5 * i + l] = d;
+      if (A.level0) {
+        r2 = d * d;
+        if (l == 0) rr = r2;
+        bad = not_finite(v) ? 1 : 0;
+      }
+    }
+  } else if (in) {
+    if (FP64) {
+      const NodePrim p = node_prim(x[0], x[1], x[2], x[3], x[4]);
+      if (l == 0) store_rec(A.rec_out, i, p);
+    } else if (DW) {
+      const NodePrimDW q = node_prim_dw(x[0], x[1], x[2], x[3], x[4]);
+      if (l == 0) store_prim_dw(A.rec2, i, q);
+    } else if (l == 0) {
+      store_rec32_from_var(A.rec32, i, x[0], x[1], x[2], x[3], x[4]);
+    }
+  }
+  if (!LAST || !A.level0) return;
+  block_norms(srms, srho, sbad, r2, rr, bad, A.st);
+}
+
 // The step-begin arrays of the level that a transfer writes, whose next
 // smoothing step begins in the transfer.
 struct BeginArgs {
@@ -1366,6 +1578,22 @@ __global__ void k_step_factors(int32_t n, int32_t off, const double* __restrict_
 // Host side.
 
 
+// The largest level that k_stage_small runs.  Above the line its eight threads
+// per node cost more issue than the shorter chains save: FP64 evaluates every
+// edge at both ends and DW passes 26 words per edge end through shared memory.
+// Measured, V-cycle with level 0 in k_stage_small against k_update, us: FP64
+// 16^3 86 / 98, 20^3 96 / 89; mixed 24^3 82 / 83, 32^3 98 / 86; DW 20^3 100.4 /
+// 100.5, 24^3 106 / 102.
+int32_t mgcfd::small_level_nodes(const mgcfd_solver* s) {
+  return s->opt.precision == MGCFD_PRECISION_FP64 ? 4096 : s->opt.precision == MGCFD_PRECISION_DW ? 8192 : 16384;
+}
+
+bool mgcfd::wants_slices(const mgcfd_solver* s, int32_t n) {
+  return s->fused ? s->fused_variant == 0 : s->small_fp64 && n <= small_level_nodes(s);
+}
+
+bool mgcfd::wants_edge_lists(const mgcfd_solver* s, int32_t n) { return s->gather || wants_slices(s, n); }
+
 namespace {
 
 int grid(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
@@ -1427,6 +1655,16 @@ const UpdateFn kUpdateFused[32] = {
     launch_update_fused<0, 0, 0, 3>, launch_update_fused<0, 0, 1, 3>, launch_update_fused<0, 1, 0, 3>,
     launch_update_fused<0, 1, 1, 3>, launch_update_fused<1, 0, 0, 3>, launch_update_fused<1, 0, 1, 3>,
     launch_update_fused<1, 1, 0, 3>, launch_update_fused<1, 1, 1, 3>};
+
+template <int P, bool L, bool Q>
+void launch_small(int64_t n, cudaStream_t st, bool chained, const UpdateArgs& A) {
+  launch(k_stage_small<P, L, Q>, grid(n, kSmallNodes), kNodeThreads, st, chained, A);
+}
+using SmallFn = void (*)(int64_t, cudaStream_t, bool, const UpdateArgs&);
+// Indexed by form (FP64, MIXED with FP64 sums, MIXED with pair sums, DW) * 2 + last.
+const SmallFn kStageSmall[8] = {launch_small<0, 0, 0>, launch_small<0, 1, 0>, launch_small<1, 0, 0>,
+                                launch_small<1, 1, 0>, launch_small<1, 0, 1>, launch_small<1, 1, 1>,
+                                launch_small<2, 0, 0>, launch_small<2, 1, 0>};
 
 template <bool M, bool S, bool W = false>
 void launch_step_begin(const DevLevel& D, unsigned long long* key, const DevStatus* st, const SegStop* ss,
@@ -1537,7 +1775,7 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
         CK(cudaEventRecord(ev.second, s->stream));
         s->pending.push_back(ev);
       }
-    } else if (D.ne > 0 && !s->fused) {
+    } else if (D.ne > 0 && !s->fused && !D.small) {
       const int g = grid(D.ne, et);
       if (dw) {
         launch(s->gather ? k_flux_dw<true> : k_flux_dw<false>, g, et, s->stream, pdl, D.ne, D.e2n, D.w4dw, D.rec2, D.flux, D.fe, s->st);
@@ -1564,7 +1802,22 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
     A.e2n = D.e2n; A.w4f = D.w4f; A.b_nbr = D.b_nbr; A.b_w4f = D.b_w4f;
     A.rec2_in = nullptr; A.off2 = D.off2; A.ent2 = D.ent2; A.w4dw = D.w4dw;
     A.sl_off = D.sl_off; A.sl_nbr = D.sl_nbr; A.sl_w = D.sl_w; A.sl_w2 = D.sl_w2;
-    if (s->fused && dw) {
+    if (D.small) {
+      // The stages' input and output records; FP64: three buffers, since a
+      // stage's blocks read their neighbours' records while others store, and
+      // the last stage stores the state into rec.
+      A.rec_in = rk == 0 ? D.rec : rk == 1 ? D.rec_s1 : D.rec_s2;
+      A.rec_out = rk == 0 ? D.rec_s1 : D.rec_s2;
+      A.rec2_in = (rk & 1) ? D.rec2b : D.rec2;
+      A.rec2 = (rk & 1) ? D.rec2 : D.rec2b;
+      A.rec32_in = (rk & 1) ? D.rec32b : D.rec32;
+      A.rec32 = (rk & 1) ? D.rec32 : D.rec32b;
+      kStageSmall[2 * (dw ? 3 : pair ? 2 : mixed ? 1 : 0) + (last ? 1 : 0)](D.n, s->stream, pdl, A);
+      if (time_this) {
+        CK(cudaEventRecord(ev.second, s->stream));
+        s->pending.push_back(ev);
+      }
+    } else if (s->fused && dw) {
       // Stage rk reads the primitives of stage rk and writes those of rk + 1
       // into the other buffer: k_step_begin fills rec2 for stage 0.
       A.rec2_in = (rk & 1) ? D.rec2b : D.rec2;
@@ -1816,51 +2069,23 @@ int colour_edges(mgcfd_solver* s, DevLevel& D) {
   return MGCFD_OK;
 }
 
-// The sliced edge lists of every level of a solver with the fused stage
-// (mixed precision without the measured-slower options, and DW), from its CSR
-// tables and weights.  A level whose slices would hold more than 1.25 entries
-// for each edge end -- its neighbouring nodes' edge counts differ much, as on a
-// random graph -- keeps the CSR lists: there the padding costs more than the
-// whole lines save.  (8192 entries are allowed on top, so that small levels,
-// whose last slice is mostly empty, are not ruled out.)
-template <class W>
+// The sliced edge lists of a solver's levels (wants_slices), from their CSR
+// tables, slice offsets and weights.  A level whose slices would hold more than
+// 1.25 entries for each edge end -- its neighbouring nodes' edge counts differ
+// much, as on a random graph -- keeps the CSR lists: there the padding costs
+// more than the whole lines save.  (8192 entries are allowed on top, so that
+// small levels, whose last slice is mostly empty, are not ruled out.)
+template <class W, bool DW>
 int build_slices(mgcfd_solver* s, W* DevLevel::*weights, W* DevLevel::*slice_weights) {
-  const size_t nl = s->L.size();
-  std::vector<int32_t> rows(nl, 0);
-  std::vector<int32_t*> off(nl, nullptr);
-  struct Scratch {
-    cudaStream_t stream;
-    std::vector<void*> p;
-    ~Scratch() { for (void* q : p) cudaFreeAsync(q, stream); }
-  } tmp{s->stream, {}};
   int r;
-  for (size_t l = 0; l < nl; l++) {
-    DevLevel& D = s->L[l];
-    if (D.n == 0 || D.ne == 0) continue;
-    const int32_t ns = (D.n + 31) / 32;
-    int32_t* width = nullptr;
-    void* t = nullptr;
-    size_t bytes = 0;
-    if ((r = s->alloc(&D.sl_off, (size_t)ns + 1))) return r;
-    CK(cudaMallocAsync(reinterpret_cast<void**>(&width), sizeof(int32_t) * ((size_t)ns + 1), s->stream));
-    tmp.p.push_back(width);
-    CK(cudaMemsetAsync(width + ns, 0, sizeof(int32_t), s->stream));
-    k_slice_width<<<grid(D.n, 256), 256, 0, s->stream>>>(D.n, D.a_off, D.b_off, width);
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, width, D.sl_off, ns + 1, s->stream));
-    CK(cudaMallocAsync(&t, bytes, s->stream));
-    tmp.p.push_back(t);
-    CK(cub::DeviceScan::ExclusiveSum(t, bytes, width, D.sl_off, ns + 1, s->stream));
-    CK(cudaMemcpyAsync(&rows[l], D.sl_off + ns, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
-  }
-  CK(cudaStreamSynchronize(s->stream));
-  for (size_t l = 0; l < nl; l++) {
-    DevLevel& D = s->L[l];
-    const int64_t entries = 32 * (int64_t)rows[l];
-    if (entries == 0 || rows[l] < 0 || entries > 2 * (int64_t)D.ne + D.ne / 2 + 8192) continue;
+  for (auto& D : s->L) {
+    const int64_t entries = 32 * (int64_t)D.sl_rows;
+    if (D.ne == 0 || entries <= 0 || entries > 2 * (int64_t)D.ne + D.ne / 2 + 8192) continue;
     if ((r = s->alloc(&(D.*slice_weights), (size_t)entries)) || (r = s->alloc(&D.sl_nbr, (size_t)entries))) return r;
     CK(cudaMemsetAsync(D.sl_nbr, 0xff, sizeof(int32_t) * (size_t)entries, s->stream));
-    k_slice_fill<W><<<grid(D.ne, 256), 256, 0, s->stream>>>(D.ne, D.e2n, D.b_list, D.a_off, D.b_off, D.*weights,
-                                                            D.sl_off, D.sl_nbr, D.*slice_weights);
+    k_slice_fill<W, DW><<<grid(D.ne, 256), 256, 0, s->stream>>>(D.ne, D.e2n, D.b_list, D.a_off, D.b_off, D.*weights,
+                                                                D.sl_off, D.sl_nbr, D.*slice_weights);
+    D.small = s->nseg == 1 && D.n <= small_level_nodes(s);
   }
   CK(cudaGetLastError());
   return MGCFD_OK;
@@ -1893,7 +2118,7 @@ int build_dw_tables(mgcfd_solver* s) {
     return set_error(MGCFD_ERR_INVALID, std::to_string(nbad) + " edge weight components outside the DW form's "
                                         "range [2^-70, 2^70); use FP64 precision for this mesh");
   if (!s->fused) return MGCFD_OK;
-  if ((r = build_slices(s, &DevLevel::w4dw, &DevLevel::sl_w2))) return r;
+  if ((r = build_slices<double4_32a, true>(s, &DevLevel::w4dw, &DevLevel::sl_w2))) return r;
   for (auto& D : s->L) {
     if ((r = s->alloc(&D.rec2b, 8 * (size_t)D.n))) return r;
     if (D.sl_nbr) continue;
@@ -1912,7 +2137,7 @@ int build_dw_tables(mgcfd_solver* s) {
 // lists, or, on a level that has none, the b-side copies in b_list order.
 int build_fused_tables(mgcfd_solver* s) {
   int r;
-  if (s->fused_variant == 0 && (r = build_slices(s, &DevLevel::w4f, &DevLevel::sl_w))) return r;
+  if ((r = build_slices<float4, false>(s, &DevLevel::w4f, &DevLevel::sl_w))) return r;
   for (auto& D : s->L) {
     if ((r = s->alloc(&D.rec32b, 8 * (size_t)D.n))) return r;
     if (D.sl_nbr) continue;
@@ -1927,7 +2152,12 @@ int build_fused_tables(mgcfd_solver* s) {
 // The tables of the solver's own form, once every level's are in place.
 int build_form_tables(mgcfd_solver* s) {
   if (s->opt.precision == MGCFD_PRECISION_DW) return build_dw_tables(s);
-  return s->fused ? build_fused_tables(s) : MGCFD_OK;
+  if (s->fused) return build_fused_tables(s);
+  if (!s->small_fp64) return MGCFD_OK;
+  int r = build_slices<double4_32a, false>(s, &DevLevel::w4, &DevLevel::sl_w2);
+  for (auto& D : s->L)
+    if (!r && D.small && !(r = s->alloc(&D.rec_s1, 8 * (size_t)D.n))) r = s->alloc(&D.rec_s2, 8 * (size_t)D.n);
+  return r;
 }
 
 // Increment strategy: AUTO is FP64 atomics for FP64, and the fused
@@ -1948,6 +2178,8 @@ int resolve_increment(mgcfd_solver* s) {
   s->coloured = inc == MGCFD_INCREMENT_COLOURED;
   s->fused = inc == MGCFD_INCREMENT_FUSED || (inc == MGCFD_INCREMENT_AUTO && (mixed || dw));
   s->gather = s->fused || inc == MGCFD_INCREMENT_GATHER;
+  // FP64 by default runs its small levels with k_stage_small (plain solvers).
+  s->small_fp64 = inc == MGCFD_INCREMENT_AUTO && s->opt.precision == MGCFD_PRECISION_FP64 && !s->opt.measure_mem_bound;
   s->fused_variant = !s->fused ? 0 : s->opt.edge_parallel_stage ? 2 : s->opt.stage_neighbour_ids ? 1 : 0;
   return MGCFD_OK;
 }
@@ -1985,6 +2217,10 @@ extern "C" int mgcfd_solver_create(int32_t nlevels, const mgcfd_level_view* leve
     s->owns_stream = true;
   }
   mgcfd_freestream_init(mach, aoa_deg, &s->ff);
+  // FP64 builds edge lists for its small levels only, about 70 us of set-up: a
+  // V-cycle of a mesh up to 32^3 nodes gains 5 to 20 us from them, a larger
+  // one's a percent or two.
+  s->small_fp64 = s->small_fp64 && levels[0].nnodes <= 32768;
 
   keep_freed_memory(s->device);
   s->L.resize((size_t)nlevels);
@@ -2033,15 +2269,26 @@ extern "C" int mgcfd_solver_create(int32_t nlevels, const mgcfd_level_view* leve
     } else {
       if ((r = s->upload(&D.w4, p.w4.data(), (size_t)p.ne))) return r;
     }
-    if (s->gather) {
+    if (wants_edge_lists(s.get(), p.n)) {
       if ((r = s->upload(&D.a_off, p.a_off.data(), (size_t)p.n + 1)) ||
           (r = s->upload(&D.b_off, p.b_off.data(), (size_t)p.n + 1)) ||
           (r = s->upload(&D.b_list, p.b_list.data(), (size_t)p.ne)))
         return r;
-      if (!s->fused && (r = mixed ? s->alloc(&D.fe32, 5 * (size_t)p.ne) : s->alloc(&D.fe, 5 * (size_t)p.ne))) return r;
-    } else {
-      if ((r = s->alloc(&D.flux, 5 * (size_t)p.n))) return r;
+      if (wants_slices(s.get(), p.n)) {
+        std::vector<int32_t> off((size_t)(p.n + 31) / 32 + 1, 0);
+        for (int32_t i = 0; i < p.n; i++) {
+          int32_t& w = off[(size_t)i / 32 + 1];
+          w = std::max(w, (p.a_off[(size_t)i + 1] - p.a_off[(size_t)i]) + (p.b_off[(size_t)i + 1] - p.b_off[(size_t)i]));
+        }
+        for (size_t k = 1; k < off.size(); k++) off[k] += off[k - 1];
+        D.sl_rows = off.back();
+        if ((r = s->upload(&D.sl_off, off.data(), off.size()))) return r;
+        CK(cudaStreamSynchronize(s->stream));  // off's host buffer
+      }
     }
+    if (!s->gather) r = s->alloc(&D.flux, 5 * (size_t)p.n);
+    else if (!s->fused) r = mixed ? s->alloc(&D.fe32, 5 * (size_t)p.ne) : s->alloc(&D.fe, 5 * (size_t)p.ne);
+    if (r) return r;
     if (s->opt.measure_mem_bound && (r = s->alloc(&D.dummy, 5 * (size_t)p.n))) return r;
     if (!p.n2mg.empty() && ((r = s->upload(&D.n2mg, p.n2mg.data(), (size_t)p.n)) ||
                             (r = s->upload(&D.dvec, p.dvec.data(), (size_t)p.n))))
@@ -2105,6 +2352,7 @@ extern "C" int mgcfd_batch_create(int32_t nmeshes, int32_t nlevels, const mgcfd_
   if (total0 > 2147483647ll) return set_error(MGCFD_ERR_INVALID, "batch too large for int32 node ids");
   s->ff = s->seg_ff[0];
   s->nseg = nmeshes;
+  s->small_fp64 = false;
   s->L.resize((size_t)nlevels);
   if ((r = device_prepare(s.get(), meshes))) return r;
   if ((r = build_form_tables(s.get()))) return r;

@@ -74,10 +74,14 @@ struct DevLevel {
   double* rec2b = nullptr;        // DW fused: second primitive buffer (stages ping-pong)
   // Fused: sliced edge lists (k_slice_fill): sl_off [slices + 1] rows of 32 entries, then per entry the
   // neighbour (bit 31: end b, -1: none) and the weights (mixed: sl_w, DW: sl_w2); null: CSR lists instead.
+  int32_t sl_rows = 0;
   int32_t* sl_off = nullptr;
   int32_t* sl_nbr = nullptr;
   float4* sl_w = nullptr;
-  double4_32a* sl_w2 = nullptr;
+  double4_32a* sl_w2 = nullptr;   // (FP64, small levels: w4)
+  bool small = false;             // k_stage_small runs this level
+  double* rec_s1 = nullptr;       // FP64 small levels: the records between the stages
+  double* rec_s2 = nullptr;
   int32_t* off2 = nullptr;        // DW fused: [N+1] each node's entries in ent2 (a_off + b_off)
   int2* ent2 = nullptr;           // DW fused: [2E] a node's a-side edges, then its b-side ones: (neighbour,
                                   // edge index, bit 31 set on the b side)
@@ -133,6 +137,7 @@ struct mgcfd_solver {
   bool begun = false;   // the next smoothing step's begin is already enqueued (by a transfer or set-up)
   bool gather = false;  // node-side CSR tables exist (GATHER or FUSED)
   bool fused = false;   // FUSED: flux and update in one node-centric kernel
+  bool small_fp64 = false;  // FP64: small levels run k_stage_small
   bool coloured = false;  // COLOURED: one flux launch per colour class, plain increments
   int fused_variant = 0;  // FUSED: 0 per-node edge loop, 1 neighbour ids staged by cp.async, 2 edge-parallel
   cudaGraphExec_t graph = nullptr;
@@ -171,6 +176,13 @@ struct mgcfd_solver {
 };
 
 namespace mgcfd {
+// The largest level that runs with eight threads per node (plain solvers).
+int32_t small_level_nodes(const mgcfd_solver* s);
+// Whether a level of n nodes needs its per-node edge lists (a_off, b_off, b_list).
+bool wants_edge_lists(const mgcfd_solver* s, int32_t n);
+// Whether they are sliced (k_slice_fill).
+bool wants_slices(const mgcfd_solver* s, int32_t n);
+
 struct MeshInput {
   const mgcfd_level_view* levels;  // s->L.size() levels
   mgcfd_freestream ff;

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import mgcfd
+from irregular import irregular_levels
 from mgcfd import _build
 
 pytestmark = pytest.mark.gpu
@@ -157,3 +158,56 @@ def test_sum32_beyond_binary32_and_not_finite(native):
     np.testing.assert_array_equal(out[4:6], [np.inf, -np.inf])  # leaves binary32's range
     assert out[6] == 0.0
     assert out[7] == float(x[7, 0]) + float(x[7, 1])
+
+
+def _small_levels(kind):
+    if kind == "irregular":  # up to fifteen or so edges at a node: two rounds of eight
+        return irregular_levels(1500, 3, 3)
+    if kind == "hub":  # one node with forty edges: five rounds and a ragged one
+        levels = irregular_levels(300, 1, 8)
+        L = levels[0]
+        e = np.stack([np.full(40, 7), np.arange(40, 80)], 1).astype(np.int32)
+        d = L.coords[e[:, 1]] - L.coords[e[:, 0]]
+        L.edge_to_nodes = np.ascontiguousarray(np.concatenate([L.edge_to_nodes, e]))
+        L.edge_weights = np.ascontiguousarray(np.concatenate([L.edge_weights, 0.02 * d]))
+        return levels
+    n = int(kind)
+    return mgcfd.HostMesh.generate(n, min(3, max(1, n.bit_length() - 1)), 70 + n).levels()
+
+
+# lattices: 8 nodes; ragged last blocks; the last level with eight threads per node and the
+# first without for FP64 (16, 17), DW (20, 21) and mixed (25, 26)
+@pytest.mark.parametrize("kind", ["2", "3", "5", "16", "17", "20", "21", "25", "26", "irregular", "hub"])
+@pytest.mark.parametrize("form", ["fp64", "mixed", "pair32", "dw"])
+def test_small_levels_equal_the_other_stage(kind, form):
+    """Small levels (eight threads per node) against the same solve with
+    k_update's stages: mixed precision against the gather increment and DW
+    against a batch of the mesh and a copy, bit for bit; FP64 against the atomic
+    increment, whose sums differ in order alone (a few 1e-16 of the state)."""
+    levels = _small_levels(kind)
+    opts = dict(precision="mixed", accumulation=form if form == "pair32" else "fp64") if form in ("mixed", "pair32") \
+        else dict(precision=form)
+
+    def solve(**more):
+        s = mgcfd.Solver(levels, 0.55, 2.5, **opts, **more)
+        s.run(2)
+        assert s.synchronize() == 0
+        out = [s.fetch(l) for l in range(len(levels))], s.norms()[1:]
+        s.close()
+        return out
+
+    got, norms = solve()
+    if form == "dw":
+        b = mgcfd.Batch([levels, levels], [0.55, 0.55], [2.5, 2.5], **opts)
+        b.run(2)
+        assert b.synchronize() == 0
+        want, wnorms = [b.fetch_mesh(1, l) for l in range(len(levels))], b.mesh_status(1)[1:]
+        b.close()
+    else:
+        want, wnorms = solve(increment="atomic" if form == "fp64" else "gather")
+    for l in range(len(levels)):
+        if form == "fp64":
+            np.testing.assert_allclose(got[l], want[l], rtol=0, atol=1e-13 * np.abs(want[l]).max())
+        else:
+            np.testing.assert_array_equal(got[l], want[l])
+    np.testing.assert_allclose(norms, wnorms, rtol=1e-6, atol=0)
