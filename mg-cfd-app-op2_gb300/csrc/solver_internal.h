@@ -112,6 +112,7 @@ struct mgcfd_solver {
   std::vector<DevLevel> L;
   std::vector<void*> allocs;
   DevStatus* st = nullptr;
+  DevStatus host_st{};  // plain solvers: *st as the last synchronize read it
   double* fetch_buf = nullptr;
   int64_t device_bytes = 0;
   // Batched solvers: nseg meshes concatenated per level (nseg == 1: plain).
