@@ -1,0 +1,37 @@
+// Launches of kernels that follow one another on a stream as programmatic
+// dependents: such a kernel begins with grid_wait, which returns when the whole
+// grid before it has finished and its writes are visible.  The order is the
+// stream's; what overlaps is the launch (and whatever the kernel does before
+// the wait, on data that no earlier kernel of the stream writes) with the
+// previous kernel's end.  After the wait, data of earlier kernels is read
+// through pointers without __restrict__: a load from a const __restrict__
+// pointer may be hoisted above the wait or take the read-only path.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace mgcfd {
+
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next kernel start its blocks before this one's exit.
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launches a kernel that begins with grid_wait as the programmatic dependent
+// of the kernel before it in the stream (`chained`), else in plain stream order.
+template <class... P, class... A>
+void launch(void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t stream, bool chained, A... args) {
+  cudaLaunchConfig_t c = {};
+  cudaLaunchAttribute at;
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = stream;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, P(args)...);  // errors: the callers' cudaGetLastError
+}
+
+}  // namespace mgcfd

@@ -12,11 +12,17 @@
 // per indirect loop: the plan-free kernels below remain for calls made while
 // plans are switched off, or while a stream captures a graph before the
 // map's plan exists.
+//
+// The V-cycle's loops are a hundred short kernels on one stream: they are
+// launched as programmatic dependents (launch.cuh), so that a launch costs
+// little more than its kernel.  Every argument is the caller's and may come
+// from the kernel before, so nothing is read before the wait.
 #include <cfloat>
 #include <cstdio>
 
 #include "common.h"
 #include "device_math.cuh"
+#include "launch.cuh"
 #include "plans.h"
 
 using namespace mgcfd;
@@ -29,6 +35,18 @@ int grid_for(int64_t n) {
   int64_t b = (n + kThreads - 1) / kThreads;
   const int64_t cap = 152 * 32;  // grid-stride loops beyond 32 blocks per SM
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
+}
+
+// Blocks of the reductions: each thread takes a run of values.
+int grid_reduce(int64_t n) {
+  const int b = grid_for(n), cap = 152 * 4;
+  return b < cap ? b : cap;
+}
+
+// A kernel that begins with grid_wait, behind the one before it on the stream.
+template <class... P, class... A>
+void chain(void (*kernel)(P...), int blocks, void* stream, A... args) {
+  launch(kernel, blocks, kThreads, static_cast<cudaStream_t>(stream), true, args...);
 }
 
 int launch_status(const char* what) {
@@ -93,13 +111,14 @@ __global__ void k_scale(int64_t n, double s, double* __restrict__ a) {
   MGCFD_GRID_STRIDE(i, n) a[i] *= s;
 }
 
-__global__ void k_copy(int64_t n, const double* __restrict__ src, double* __restrict__ dst) {
+__global__ void k_copy(int64_t n, const double* src, double* dst) {
+  grid_wait();
   MGCFD_GRID_STRIDE(i, n) dst[i] = src[i];
 }
 
 // time_stepping_kernels.h:13-32
-__global__ void k_calculate_dt(int32_t n, const double* __restrict__ var, const double* __restrict__ vol,
-                               double* __restrict__ dt) {
+__global__ void k_calculate_dt(int32_t n, const double* var, const double* vol, double* dt) {
+  grid_wait();
   MGCFD_GRID_STRIDE(i, n) {
     const double* x = var + 5 * i;
     NodePrim p = node_prim(x[0], x[1], x[2], x[3], x[4]);
@@ -107,39 +126,41 @@ __global__ void k_calculate_dt(int32_t n, const double* __restrict__ var, const 
   }
 }
 
-__global__ void k_set_scalar(double* p, double v) { *p = v; }
-
-// Block minimum, then one compare-and-swap loop per block on the double.
-__device__ void atomic_min_double(double* addr, double v) {
-  unsigned long long* a = reinterpret_cast<unsigned long long*>(addr);
-  unsigned long long old = *a;
-  while (v < __longlong_as_double((long long)old)) {
-    unsigned long long assumed = old;
-    old = atomicCAS(a, assumed, (unsigned long long)__double_as_longlong(v));
-    if (old == assumed) break;
-  }
+__global__ void k_set_scalar(double* p, double v) {
+  grid_wait();
+  *p = v;
 }
 
-__global__ void k_min_dt(int32_t n, const double* __restrict__ dt, double* __restrict__ out) {
-  __shared__ double sm[kThreads / 32];
-  double m = DBL_MAX;
+// get_min_dt_kernel over order-preserving integer keys (dt_candidate_key: NaN
+// never replaces DBL_MAX), so the reduction issues no FP64 compare, in few
+// enough blocks that their atomics do not queue: 17 us with FP64 compares and
+// a compare-and-swap loop per 256 nodes at 1M nodes, for 8 MB of dt.  The
+// combination is an integer atomic on the double itself: values >= 0 order as
+// signed integers, below 0 as unsigned ones reversed, and below 0 wins.
+__global__ void __launch_bounds__(kThreads) k_min_dt(int32_t n, const double* dt, double* out) {
+  __shared__ unsigned long long sm[kThreads / 32];
+  grid_wait();
+  unsigned long long m = ~0ull;
   MGCFD_GRID_STRIDE(i, n) {
-    const double v = dt[i];
-    if (v < m) m = v;  // NaN never replaces, as in get_min_dt_kernel
+    const unsigned long long k = dt_candidate_key(dt[i]);
+    m = k < m ? k : m;
   }
-  m = warp_min(m);
+  m = warp_min_u64(m);
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
   __syncthreads();
   if (threadIdx.x < 32) {
-    m = threadIdx.x < kThreads / 32 ? sm[threadIdx.x] : DBL_MAX;
-    m = warp_min(m);
-    if (threadIdx.x == 0 && m < DBL_MAX) atomic_min_double(out, m);
+    m = warp_min_u64(threadIdx.x < kThreads / 32 ? sm[threadIdx.x] : ~0ull);
+    if (threadIdx.x == 0 && m != ~0ull) {
+      const unsigned long long bits = (m >> 63) ? (m & 0x7fffffffffffffffull) : ~m;
+      if (bits >> 63) atomicMax(reinterpret_cast<unsigned long long*>(out), bits);
+      else atomicMin(reinterpret_cast<long long*>(out), (long long)bits);
+    }
   }
 }
 
 // time_stepping_kernels.h:43-64 (only the final division matters).
-__global__ void k_step_factor(int32_t n, const double* __restrict__ vol, const double* __restrict__ min_dt,
-                              double* __restrict__ sf) {
+__global__ void k_step_factor(int32_t n, const double* vol, const double* min_dt, double* sf) {
+  grid_wait();
   const double m = *min_dt;
   MGCFD_GRID_STRIDE(i, n) sf[i] = div_fast(m, vol[i]);
 }
@@ -169,17 +190,17 @@ __global__ void k_flux_edge(int32_t ne, int32_t nn, const int32_t* __restrict__ 
 }
 
 // flux.h:14-39 over boundary entries.
-__global__ void k_bnd_flux(int32_t nb, int32_t nn, const int32_t* __restrict__ b2n, const int32_t* __restrict__ grp,
-                           const double* __restrict__ bw, const double* __restrict__ var, mgcfd_freestream ff,
-                           double* __restrict__ flux) {
+__global__ void k_bnd_flux(int32_t nb, int32_t nn, const int32_t* b2n, const int32_t* grp, const double* bw,
+                           const double* var, mgcfd_freestream ff, double* flux) {
+  grid_wait();
   MGCFD_GRID_STRIDE(i, nb) {
     const int g = grp[i];
-    if (g > 7) continue;
     const int32_t n = b2n[i];
+    const double wx = bw[3 * i], wy = bw[3 * i + 1], wz = bw[3 * i + 2];
+    if (g > 7) continue;
     if (!in_range(n, nn)) { map_error(); continue; }
     const double* x = var + 5 * (int64_t)n;
     const NodePrim b = node_prim(x[0], x[1], x[2], x[3], x[4]);
-    const double wx = bw[3 * i], wy = bw[3 * i + 1], wz = bw[3 * i + 2];
     double* fb = flux + 5 * (int64_t)n;
     if (g <= 2) {
       atomicAdd(fb + 1, wx * b.p);
@@ -208,8 +229,8 @@ __global__ void k_bnd_flux(int32_t nb, int32_t nn, const int32_t* __restrict__ b
 // access of the [N][5] dats is coalesced (a thread per node reads rows 40 B
 // apart, five times per array: measured 1.06 ms at 8M nodes against the
 // 0.2 ms its bytes need).
-__global__ void k_time_step(int64_t n5, double inv_div, const double* __restrict__ sf, double* __restrict__ flux,
-                            const double* __restrict__ old, double* __restrict__ var) {
+__global__ void k_time_step(int64_t n5, double inv_div, const double* sf, double* flux, const double* old, double* var) {
+  grid_wait();
   MGCFD_GRID_STRIDE(j, n5) {
     const double factor = sf[j / 5] * inv_div;
     var[j] = old[j] + factor * flux[j];
@@ -241,21 +262,28 @@ __global__ void k_stream(int32_t ne, int32_t nn, const int32_t* __restrict__ e2n
   }
 }
 
-__global__ void k_residual(int64_t n, const double* __restrict__ old, const double* __restrict__ var,
-                           double* __restrict__ res) {
+__global__ void k_residual(int64_t n, const double* old, const double* var, double* res) {
+  grid_wait();
   MGCFD_GRID_STRIDE(i, n) res[i] = var[i] - old[i];
 }
 
-__global__ void k_sum_squares(int64_t n, const double* __restrict__ x, double* __restrict__ out) {
-  __shared__ double sm[kThreads / 32];
+// calc_rms_kernel: the block's sum by halving the active threads through
+// shared memory, so nearly every FP64 add is a useful one, and few enough
+// blocks that each thread sums a run (a shuffle tree per 256 values issued as
+// many FP64 adds again: 26 us at 1M nodes for 40 MB).
+__global__ void __launch_bounds__(kThreads) k_sum_squares(int64_t n, const double* x, double* out) {
+  __shared__ double sm[kThreads];
+  grid_wait();
   double s = 0.0;
   MGCFD_GRID_STRIDE(i, n) s += x[i] * x[i];
-  s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  sm[threadIdx.x] = s;
   __syncthreads();
+  for (int w = kThreads / 2; w >= 32; w >>= 1) {
+    if ((int)threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
+    __syncthreads();
+  }
   if (threadIdx.x < 32) {
-    s = threadIdx.x < kThreads / 32 ? sm[threadIdx.x] : 0.0;
-    s = warp_sum(s);
+    s = warp_sum(sm[threadIdx.x]);
     if (threadIdx.x == 0) atomicAdd(out, s);
   }
 }
@@ -272,12 +300,10 @@ __device__ __forceinline__ void block_add_int(int c, int32_t* out) {
   }
 }
 
-__global__ void k_count_bad(int64_t n, const double* __restrict__ x, int32_t* __restrict__ out) {
+__global__ void k_count_bad(int64_t n, const double* x, int32_t* out) {
+  grid_wait();
   int c = 0;
-  MGCFD_GRID_STRIDE(i, n) {
-    const double v = x[i];
-    if (isnan(v) || isinf(v)) c++;
-  }
+  MGCFD_GRID_STRIDE(i, n) c += not_finite(x[i]) ? 1 : 0;  // from the exponent field: no FP64 compare
   block_add_int(c, out);
 }
 
@@ -317,10 +343,11 @@ __global__ void k_up(int32_t nf, int32_t nc, const int32_t* __restrict__ map, co
     atomicAdd(scratch + c, 1);
   }
 }
-__global__ void k_up_post(int32_t nc, double* __restrict__ cv, const int32_t* __restrict__ scratch) {
+__global__ void k_up_post(int32_t nc, double* cv, const int32_t* scratch) {
+  grid_wait();
   MGCFD_GRID_STRIDE(i, nc) {
     const int32_t s = scratch[i];
-    const double avg = s == 0 ? 1.0 : 1.0 / (double)s;
+    const double avg = s == 0 ? 1.0 : rcp_fast((double)s);
 #pragma unroll
     for (int k = 0; k < 5; k++) cv[5 * i + k] *= avg;
   }
@@ -329,20 +356,27 @@ __global__ void k_up_post(int32_t nc, double* __restrict__ cv, const int32_t* __
 // mg.h:66-88.  (Staging the fine rows through shared memory for coalesced
 // access measured slower here, 0.78 against 0.39 ms at 8M nodes: the gathers
 // of the coarse rows are latency-bound and the staging barriers expose them.)
-__global__ void k_down(int32_t nf, int32_t nc, const int32_t* __restrict__ map, double* __restrict__ fv,
-                       const double* __restrict__ fres, const double* __restrict__ fx,
-                       const double* __restrict__ cres, const double* __restrict__ cx) {
+__global__ void k_down(int32_t nf, int32_t nc, const int32_t* map, double* fv, const double* fres, const double* fx,
+                       const double* cres, const double* cx) {
+  grid_wait();
   MGCFD_GRID_STRIDE(i, nf) {
     const int32_t ci = map[i];
+    double v[5], r[5], x[3];
+#pragma unroll
+    for (int k = 0; k < 5; k++) { v[k] = fv[5 * i + k]; r[k] = fres[5 * i + k]; }
+#pragma unroll
+    for (int k = 0; k < 3; k++) x[k] = fx[3 * i + k];
     if (!in_range(ci, nc)) { map_error(); continue; }
     const int64_t c = ci;
-    const double dx = fabs(fx[3 * i] - cx[3 * c]);
-    const double dy = fabs(fx[3 * i + 1] - cx[3 * c + 1]);
-    const double dz = fabs(fx[3 * i + 2] - cx[3 * c + 2]);
-    const double dm = sqrt(dx * dx + dy * dy + dz * dz);
+    const double dx = fabs(x[0] - cx[3 * c]);
+    const double dy = fabs(x[1] - cx[3 * c + 1]);
+    const double dz = fabs(x[2] - cx[3 * c + 2]);
+    const double dm = sqrt_fast(dx * dx + dy * dy + dz * dz);
     const double d[5] = {dm, dx, dy, dz, dm};
 #pragma unroll
-    for (int k = 0; k < 5; k++) fv[5 * i + k] -= d[k] * (cres[5 * c + k] - fres[5 * i + k]);
+    for (int k = 0; k < 5; k++) v[k] -= d[k] * (cres[5 * c + k] - r[k]);
+#pragma unroll
+    for (int k = 0; k < 5; k++) fv[5 * i + k] = v[k];
   }
 }
 
@@ -398,7 +432,7 @@ extern "C" int mgcfd_op_copy_double(int32_t n, const double* v, double* old, voi
   CHECK_N(n, "mgcfd_op_copy_double");
   CHECK_PTR(v, n, "copy_double"); CHECK_PTR(old, n, "copy_double");
   if (n == 0) return MGCFD_OK;
-  k_copy<<<grid_for(5 * (int64_t)n), kThreads, 0, STREAM(s)>>>(5 * (int64_t)n, v, old);
+  chain(k_copy, grid_for(5 * (int64_t)n), s, 5 * (int64_t)n, v, old);
   return launch_status("copy_double");
 }
 
@@ -410,7 +444,7 @@ extern "C" int mgcfd_op_calculate_dt(int32_t n, const double* v, const double* v
   int r = vol_plan_get(vol, n, STREAM(s), &plan);
   if (r) return r;
   if (plan) return vol_plan_calculate_dt(plan, v, vol, dt, STREAM(s));
-  k_calculate_dt<<<grid_for(n), kThreads, 0, STREAM(s)>>>(n, v, vol, dt);
+  chain(k_calculate_dt, grid_for(n), s, n, v, vol, dt);
   return launch_status("calculate_dt");
 }
 
@@ -418,8 +452,8 @@ extern "C" int mgcfd_op_get_min_dt(int32_t n, const double* dt, double* min_dt, 
   CHECK_N(n, "mgcfd_op_get_min_dt");
   CHECK_PTR(dt, n, "get_min_dt");
   if (!min_dt) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_get_min_dt: null output");
-  k_set_scalar<<<1, 1, 0, STREAM(s)>>>(min_dt, DBL_MAX);
-  if (n > 0) k_min_dt<<<grid_for(n), kThreads, 0, STREAM(s)>>>(n, dt, min_dt);
+  launch(k_set_scalar, 1, 1, STREAM(s), true, min_dt, DBL_MAX);
+  if (n > 0) chain(k_min_dt, grid_reduce(n), s, n, dt, min_dt);
   return launch_status("get_min_dt");
 }
 
@@ -430,7 +464,7 @@ extern "C" int mgcfd_op_compute_step_factor(int32_t n, const double* v, const do
   CHECK_PTR(vol, n, "compute_step_factor"); CHECK_PTR(sf, n, "compute_step_factor");
   if (!min_dt) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_compute_step_factor: null min_dt");
   if (n == 0) return MGCFD_OK;
-  k_step_factor<<<grid_for(n), kThreads, 0, STREAM(s)>>>(n, vol, min_dt, sf);
+  chain(k_step_factor, grid_for(n), s, n, vol, min_dt, sf);
   return launch_status("compute_step_factor");
 }
 
@@ -464,7 +498,7 @@ extern "C" int mgcfd_op_compute_bnd_node_flux(int32_t nb, int32_t nn, const int3
   CHECK_PTR(flux, nb, "compute_bnd_node_flux");
   if (!ff) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_compute_bnd_node_flux: null freestream");
   if (nb == 0) return MGCFD_OK;
-  k_bnd_flux<<<grid_for(nb), kThreads, 0, STREAM(s)>>>(nb, nn, b2n, grp, bw, v, *ff, flux);
+  chain(k_bnd_flux, grid_for(nb), s, nb, nn, b2n, grp, bw, v, *ff, flux);
   return launch_status("compute_bnd_node_flux");
 }
 
@@ -477,7 +511,7 @@ extern "C" int mgcfd_op_time_step(int32_t n, int32_t rk, const double* sf, doubl
   if (n == 0) return MGCFD_OK;
   // factor = sf / (RK + 1 - rk): divisors 4, 3, 2 become multiplications.
   const double inv_div = 1.0 / (double)(kRK + 1 - rk);
-  k_time_step<<<grid_for(5 * (int64_t)n), kThreads, 0, STREAM(s)>>>(5 * (int64_t)n, inv_div, sf, flux, old, v);
+  chain(k_time_step, grid_for(5 * (int64_t)n), s, 5 * (int64_t)n, inv_div, sf, flux, old, v);
   return launch_status("time_step");
 }
 
@@ -496,7 +530,7 @@ extern "C" int mgcfd_op_residual(int32_t n, const double* old, const double* v, 
   CHECK_N(n, "mgcfd_op_residual");
   CHECK_PTR(old, n, "residual"); CHECK_PTR(v, n, "residual"); CHECK_PTR(res, n, "residual");
   if (n == 0) return MGCFD_OK;
-  k_residual<<<grid_for(5 * (int64_t)n), kThreads, 0, STREAM(s)>>>(5 * (int64_t)n, old, v, res);
+  chain(k_residual, grid_for(5 * (int64_t)n), s, 5 * (int64_t)n, old, v, res);
   return launch_status("residual");
 }
 
@@ -505,7 +539,7 @@ extern "C" int mgcfd_op_calc_rms(int32_t n, const double* res, double* rms, void
   CHECK_PTR(res, n, "calc_rms");
   if (!rms) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_calc_rms: null output");
   if (n == 0) return MGCFD_OK;
-  k_sum_squares<<<grid_for(5 * (int64_t)n), kThreads, 0, STREAM(s)>>>(5 * (int64_t)n, res, rms);
+  chain(k_sum_squares, grid_reduce(5 * (int64_t)n), s, 5 * (int64_t)n, res, rms);
   return launch_status("calc_rms");
 }
 
@@ -514,7 +548,7 @@ extern "C" int mgcfd_op_count_bad_vals(int32_t n, const double* v, int32_t* coun
   CHECK_PTR(v, n, "count_bad_vals");
   if (!count) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_count_bad_vals: null output");
   if (n == 0) return MGCFD_OK;
-  k_count_bad<<<grid_for(5 * (int64_t)n), kThreads, 0, STREAM(s)>>>(5 * (int64_t)n, v, count);
+  chain(k_count_bad, grid_reduce(5 * (int64_t)n), s, 5 * (int64_t)n, v, count);
   return launch_status("count_bad_vals");
 }
 
@@ -570,7 +604,7 @@ extern "C" int mgcfd_op_up_post(int32_t nc, double* cv, const int32_t* scratch, 
   CHECK_N(nc, "mgcfd_op_up_post");
   CHECK_PTR(cv, nc, "up_post"); CHECK_PTR(scratch, nc, "up_post");
   if (nc == 0) return MGCFD_OK;
-  k_up_post<<<grid_for(nc), kThreads, 0, STREAM(s)>>>(nc, cv, scratch);
+  chain(k_up_post, grid_for(nc), s, nc, cv, scratch);
   return launch_status("up_post");
 }
 
@@ -581,7 +615,7 @@ extern "C" int mgcfd_op_down(int32_t nf, int32_t nc, const int32_t* map, double*
   CHECK_PTR(map, nf, "down"); CHECK_PTR(fv, nf, "down"); CHECK_PTR(fres, nf, "down"); CHECK_PTR(fx, nf, "down");
   CHECK_PTR(cres, nf, "down"); CHECK_PTR(cx, nf, "down");
   if (nf == 0) return MGCFD_OK;
-  k_down<<<grid_for(nf), kThreads, 0, STREAM(s)>>>(nf, nc, map, fv, fres, fx, cres, cx);
+  chain(k_down, grid_for(nf), s, nf, nc, map, fv, fres, fx, cres, cx);
   return launch_status("down");
 }
 

@@ -59,6 +59,7 @@
 #include "common.h"
 #include "device_math.cuh"
 #include "dw_math.cuh"
+#include "launch.cuh"
 #include "plans.h"
 #include "solver_internal.h"
 
@@ -314,13 +315,19 @@ __global__ void k_fill_u64(int64_t n, unsigned long long v, unsigned long long* 
 
 // ---- edge plan kernels -------------------------------------------------------
 
-// Primitives of every node in internal order.
+// Primitives of every node in internal order.  PERM: also clears the internal
+// increments that the flux kernel adds to.
 template <bool PERM>
-__global__ void __launch_bounds__(kT) k_plan_prims(int32_t nn, const int32_t* __restrict__ perm,
-                                                   const double* __restrict__ var, double* __restrict__ rec) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kT) k_plan_prims(int32_t nn, const int32_t* __restrict__ perm, const double* var,
+                                                   double* rec, double* fl) {
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + threadIdx.x;
+  const int64_t c = PERM && i < nn ? (int64_t)perm[i] : i;
+  grid_wait();
+  if (PERM) {
+    const int64_t end = 5 * (i0 + blockDim.x < nn ? i0 + blockDim.x : (int64_t)nn);
+    for (int64_t k = 5 * i0 + threadIdx.x; k < end; k += blockDim.x) fl[k] = 0.0;
+  }
   if (i >= nn) return;
-  const int64_t c = PERM ? (int64_t)perm[i] : i;
   const double* x = var + 5 * c;
   const NodePrim p = node_prim(x[0], x[1], x[2], x[3], x[4]);
   double4_32a* r = reinterpret_cast<double4_32a*>(rec + 8 * i);
@@ -350,13 +357,15 @@ __device__ __forceinline__ bool half_bits(double w, bool pos, unsigned long long
 // the memo when the caller's weight has the bits it was made from.
 template <bool PERM>
 __global__ void __launch_bounds__(128) k_plan_flux(int32_t ne, const int2* __restrict__ e2n,
-                                                   const int32_t* __restrict__ eref, const double* __restrict__ ewt,
-                                                   double4_32a* __restrict__ memo, int memo_valid, double sc,
-                                                   const double* __restrict__ rec, double* __restrict__ acc) {
+                                                   const int32_t* __restrict__ eref, const double* ewt,
+                                                   double4_32a* memo, int memo_valid, double sc, const double* rec,
+                                                   double* acc) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const int2 ab = e2n[e];
-  const int32_t r = eref[e];
+  const bool live = e < ne;
+  const int2 ab = live ? e2n[e] : make_int2(0, 0);
+  const int32_t r = live ? eref[e] : 0;
+  grid_wait();
+  if (!live) return;
   const bool flip = r < 0;
   const int64_t ce = flip ? (int64_t)~r : (int64_t)r;
   const double wx = ewt[3 * ce], wy = ewt[3 * ce + 1], wz = ewt[3 * ce + 2];
@@ -370,10 +379,10 @@ __global__ void __launch_bounds__(128) k_plan_flux(int32_t ne, const int2* __res
     const double h = flip ? 0.5 : -0.5;
     const double mag = sqrt(fma(wz, wz, fma(wy, wy, wx * wx)));
     m = make_double4_32a(h * wx, h * wy, h * wz, -(mag * sc) * 0.5);
-    memo[e] = m;
   }
   const NodePrim a = plan_rec(rec, ab.x);
   const NodePrim b = plan_rec(rec, ab.y);
+  if (!hit) memo[e] = m;
   double f[5];
   edge_flux(a, b, m.x, m.y, m.z, m.w, f);
   double* fa = acc + 5 * (int64_t)ab.x;
@@ -389,12 +398,12 @@ __global__ void __launch_bounds__(128) k_plan_flux(int32_t ne, const int2* __res
 // node, variable), so the caller's flux is read and written coalesced and
 // only the internal rows are gathered (five neighbouring threads share a
 // row).  A bijection: no atomics.
-__global__ void k_plan_gather(int64_t n5, const int32_t* __restrict__ pos, const double* __restrict__ fl,
-                              double* __restrict__ flux) {
+__global__ void k_plan_gather(int64_t n5, const int32_t* __restrict__ pos, const double* fl, double* flux) {
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n5) return;
   const int64_t c = j / 5;
-  flux[j] += fl[5 * (int64_t)pos[c] + (j - 5 * c)];
+  const int32_t p = j < n5 ? pos[c] : 0;
+  grid_wait();
+  if (j < n5) flux[j] += fl[5 * (int64_t)p + (j - 5 * c)];
 }
 
 // ---- edge plan, DW form ---------------------------------------------------------
@@ -457,12 +466,11 @@ __global__ void k_inv_e(int32_t nv, const int32_t* __restrict__ eref, int32_t* _
 // every edge, after a change of smoothing coefficient) gets its (h, wfac)
 // recomputed -- the FP64 plan's formula -- and stored as pair words at its
 // internal position.  Unchanged weights cost a compare.
-__global__ void k_plan_weights_dw(int32_t ne, const int32_t* __restrict__ inv, const double* __restrict__ ewt,
-                                  double* __restrict__ wcopy, double4_32a* __restrict__ memo_dw, int force,
-                                  double sc) {
+__global__ void k_plan_weights_dw(int32_t ne, const int32_t* __restrict__ inv, const double* ewt, double* wcopy,
+                                  double4_32a* memo_dw, int force, double sc) {
   const int64_t ce = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (ce >= ne) return;
-  const int32_t r = inv[ce];
+  const int32_t r = ce < ne ? inv[ce] : kNoEdge;
+  grid_wait();
   if (r == kNoEdge) return;
   const double wx = ewt[3 * ce], wy = ewt[3 * ce + 1], wz = ewt[3 * ce + 2];
   double* c = wcopy + 3 * ce;
@@ -482,11 +490,13 @@ __global__ void k_plan_weights_dw(int32_t ne, const int32_t* __restrict__ inv, c
 
 // Pair-word primitives of every node in internal order (no FP64 instruction).
 template <bool PERM>
-__global__ void __launch_bounds__(kT) k_plan_prims_dw(int32_t nn, const int32_t* __restrict__ perm,
-                                                      const double* __restrict__ var, double* __restrict__ rec2) {
+__global__ void __launch_bounds__(kT) k_plan_prims_dw(int32_t nn, const int32_t* __restrict__ perm, const double* var,
+                                                      double* rec2) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t c = PERM && i < nn ? (int64_t)perm[i] : i;
+  grid_wait();
   if (i >= nn) return;
-  const double* x = var + 5 * (PERM ? (int64_t)perm[i] : i);
+  const double* x = var + 5 * c;
   store_prim_dw(rec2, i, node_prim_dw(x[0], x[1], x[2], x[3], x[4]));
 }
 
@@ -497,17 +507,19 @@ __global__ void __launch_bounds__(kT) k_plan_prims_dw(int32_t nn, const int32_t*
 template <bool PERM>
 __global__ void __launch_bounds__(128, 8) k_plan_flux_dw(int32_t nn, const int32_t* __restrict__ perm,
                                                          const int32_t* __restrict__ off2,
-                                                         const int2* __restrict__ ent2,
-                                                         const double4_32a* __restrict__ memo_dw,
-                                                         const double* __restrict__ rec2, double* __restrict__ flux) {
+                                                         const int2* __restrict__ ent2, const double4_32a* memo_dw,
+                                                         const double* rec2, double* flux) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t k0 = i < nn ? off2[i] : 0, k1 = i < nn ? off2[i + 1] : 0;
+  int2 next = k0 < k1 ? ent2[k0] : make_int2(0, 0);
+  grid_wait();
   if (i >= nn) return;
   const dwf s_me = dw_unpack(rec2[8 * i + 6]);
   NodeFluxDW acc;
   node_flux_dw_init(acc);
-  const int32_t k0 = off2[i], k1 = off2[i + 1];
   for (int32_t j = k0; j < k1; j++) {
-    const int2 en = ent2[j];
+    const int2 en = next;  // the following entry loads during this edge's arithmetic
+    if (j + 1 < k1) next = ent2[j + 1];
     const NodePrimDW o = load_prim_dw(rec2, en.x);
     const double4_32a w = memo_dw[en.y & 0x7fffffff];
     const uint32_t sg = (uint32_t)en.y & 0x80000000u;
@@ -540,10 +552,11 @@ __global__ void k_child_pairs(int32_t nf, int32_t nc, const int32_t* __restrict_
 }
 
 // up_pre_kernel (mg.h:29-39): every coarse node with a child starts from zero.
-__global__ void k_child_pre(int32_t nc, const int32_t* __restrict__ off, double* __restrict__ cv,
-                            int32_t* __restrict__ scratch) {
+__global__ void k_child_pre(int32_t nc, const int32_t* __restrict__ off, double* cv, int32_t* scratch) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc || off[c + 1] == off[c]) return;
+  const bool children = c < nc && off[c + 1] != off[c];
+  grid_wait();
+  if (!children) return;
 #pragma unroll
   for (int k = 0; k < 5; k++) cv[5 * c + k] = 0.0;
   scratch[c] = 0;
@@ -552,10 +565,10 @@ __global__ void k_child_pre(int32_t nc, const int32_t* __restrict__ off, double*
 // up_kernel (mg.h:41-52) as a gather: the children's states added to the
 // coarse state in child order, and the count raised by the number of children.
 __global__ void k_child_up(int32_t nc, const int32_t* __restrict__ off, const int32_t* __restrict__ list,
-                           const double* __restrict__ fv, double* __restrict__ cv, int32_t* __restrict__ scratch) {
+                           const double* fv, double* cv, int32_t* scratch) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  const int32_t lo = off[c], hi = off[c + 1];
+  const int32_t lo = c < nc ? off[c] : 0, hi = c < nc ? off[c + 1] : 0;
+  grid_wait();
   if (hi == lo) return;
   double s[5];
 #pragma unroll
@@ -847,22 +860,22 @@ int build_child_plan(const int32_t* map, int32_t nf, int32_t nc, cudaStream_t s,
 // cube root taken from the plan while the volume keeps the bits it had when
 // the root was taken (a bit compare per node), else computed and kept: the
 // same bits as cbrt on every call.  node_prim and the division stay per call.
-__global__ void k_plan_calculate_dt(int32_t n, const double* __restrict__ var, const double* __restrict__ vol,
-                                    double* __restrict__ vcopy, double* __restrict__ root, double* __restrict__ dt) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = vol[i];
-    double c;
-    if (__double_as_longlong(v) == __double_as_longlong(vcopy[i])) {
-      c = root[i];
-    } else {
-      c = cbrt(v);
-      root[i] = c;
-      vcopy[i] = v;
-    }
-    const double* x = var + 5 * i;
-    const NodePrim p = node_prim(x[0], x[1], x[2], x[3], x[4]);
-    dt[i] = 0.5 * div_fast(c, p.s);
+__global__ void k_plan_calculate_dt(int32_t n, const double* var, const double* vol, double* vcopy, double* root,
+                                    double* dt) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_wait();
+  if (i >= n) return;
+  const double v = vol[i], was = vcopy[i];
+  double c = root[i];
+  const double* x = var + 5 * i;
+  const double x0 = x[0], x1 = x[1], x2 = x[2], x3 = x[3], x4 = x[4];
+  if (__double_as_longlong(v) != __double_as_longlong(was)) {
+    c = cbrt(v);
+    root[i] = c;
+    vcopy[i] = v;
   }
+  const NodePrim p = node_prim(x0, x1, x2, x3, x4);
+  dt[i] = 0.5 * div_fast(c, p.s);
 }
 
 // A volume plan starts with every copied volume and root set to the
@@ -939,33 +952,24 @@ int edge_plan_flux(EdgePlan* P, const double* var, const double* ewt, double sc,
     const bool force = !(P->memo_dw_sc == sc);  // the first DW call (NaN) or a new smoothing coefficient
     P->memo_dw_sc = sc;
     if (P->nvalid > 0)
-      k_plan_weights_dw<<<grid(P->ne), kT, 0, s>>>(P->ne, P->inv_e, ewt, P->wcopy, P->memo_dw, force ? 1 : 0, sc);
-    if (P->permuted) {
-      k_plan_prims_dw<true><<<grid(P->nn), kT, 0, s>>>(P->nn, P->perm, var, P->rec2);
-      k_plan_flux_dw<true><<<grid(P->nn, 128), 128, 0, s>>>(P->nn, P->perm, P->off2, P->ent2, P->memo_dw, P->rec2, flux);
-    } else {
-      k_plan_prims_dw<false><<<grid(P->nn), kT, 0, s>>>(P->nn, nullptr, var, P->rec2);
-      k_plan_flux_dw<false><<<grid(P->nn, 128), 128, 0, s>>>(P->nn, nullptr, P->off2, P->ent2, P->memo_dw, P->rec2,
-                                                            flux);
-    }
+      launch(k_plan_weights_dw, grid(P->ne), kT, s, true, P->ne, P->inv_e, ewt, P->wcopy, P->memo_dw, force ? 1 : 0, sc);
+    launch(P->permuted ? k_plan_prims_dw<true> : k_plan_prims_dw<false>, grid(P->nn), kT, s, true, P->nn, P->perm, var,
+           P->rec2);
+    launch(P->permuted ? k_plan_flux_dw<true> : k_plan_flux_dw<false>, grid(P->nn, 128), 128, s, true, P->nn, P->perm,
+           P->off2, P->ent2, P->memo_dw, P->rec2, flux);
     CK(cudaGetLastError());
     return MGCFD_OK;
   }
   const bool memo_valid = P->memo_sc == sc;  // false for NaN: never used yet
   P->memo_sc = sc;
-  if (P->permuted) {
-    CK(cudaMemsetAsync(P->fl, 0, sizeof(double) * 5 * (size_t)P->nn, s));
-    k_plan_prims<true><<<grid(P->nn), kT, 0, s>>>(P->nn, P->perm, var, P->rec);
-    if (P->nvalid > 0)
-      k_plan_flux<true><<<grid(P->nvalid, 128), 128, 0, s>>>(P->nvalid, P->e2n, P->eref, ewt, P->memo,
-                                                             memo_valid ? 1 : 0, sc, P->rec, P->fl);
-    k_plan_gather<<<grid(5 * (int64_t)P->nn), kT, 0, s>>>(5 * (int64_t)P->nn, P->pos, P->fl, flux);
-  } else {
-    k_plan_prims<false><<<grid(P->nn), kT, 0, s>>>(P->nn, nullptr, var, P->rec);
-    if (P->nvalid > 0)
-      k_plan_flux<false><<<grid(P->nvalid, 128), 128, 0, s>>>(P->nvalid, P->e2n, P->eref, ewt, P->memo,
-                                                              memo_valid ? 1 : 0, sc, P->rec, flux);
-  }
+  double* acc = P->permuted ? P->fl : flux;
+  launch(P->permuted ? k_plan_prims<true> : k_plan_prims<false>, grid(P->nn), kT, s, true, P->nn, P->perm, var, P->rec,
+         P->fl);
+  if (P->nvalid > 0)
+    launch(P->permuted ? k_plan_flux<true> : k_plan_flux<false>, grid(P->nvalid, 128), 128, s, true, P->nvalid, P->e2n,
+           P->eref, ewt, P->memo, memo_valid ? 1 : 0, sc, P->rec, acc);
+  if (P->permuted)
+    launch(k_plan_gather, grid(5 * (int64_t)P->nn), kT, s, true, 5 * (int64_t)P->nn, P->pos, P->fl, flux);
   CK(cudaGetLastError());
   return MGCFD_OK;
 }
@@ -979,14 +983,14 @@ int child_plan_get(const int32_t* map, int32_t nf, int32_t nc, cudaStream_t s, C
 
 int child_plan_up_pre(ChildPlan* P, double* cv, int32_t* scratch, cudaStream_t s, int64_t* skipped) {
   *skipped = P->nbad;
-  if (P->nc > 0) k_child_pre<<<grid(P->nc), kT, 0, s>>>(P->nc, P->ch_off, cv, scratch);
+  if (P->nc > 0) launch(k_child_pre, grid(P->nc), kT, s, true, P->nc, P->ch_off, cv, scratch);
   CK(cudaGetLastError());
   return MGCFD_OK;
 }
 
 int child_plan_up(ChildPlan* P, const double* fv, double* cv, int32_t* scratch, cudaStream_t s, int64_t* skipped) {
   *skipped = P->nbad;
-  if (P->nc > 0) k_child_up<<<grid(P->nc, 128), 128, 0, s>>>(P->nc, P->ch_off, P->ch_list, fv, cv, scratch);
+  if (P->nc > 0) launch(k_child_up, grid(P->nc, 128), 128, s, true, P->nc, P->ch_off, P->ch_list, fv, cv, scratch);
   CK(cudaGetLastError());
   return MGCFD_OK;
 }
@@ -1001,7 +1005,7 @@ int vol_plan_get(const double* vol, int32_t n, cudaStream_t s, VolPlan** out) {
 }
 
 int vol_plan_calculate_dt(VolPlan* P, const double* var, const double* vol, double* dt, cudaStream_t s) {
-  if (P->n > 0) k_plan_calculate_dt<<<grid(P->n), kT, 0, s>>>(P->n, var, vol, P->vcopy, P->root, dt);
+  if (P->n > 0) launch(k_plan_calculate_dt, grid(P->n), kT, s, true, P->n, var, vol, P->vcopy, P->root, dt);
   CK(cudaGetLastError());
   return MGCFD_OK;
 }

@@ -41,19 +41,13 @@
 // smoothed (get_min_dt's DBL_MAX start), and under a stop rule k_cycle_end
 // after each V-cycle.
 //
-// These launches follow one another as programmatic dependents: each loads
-// what set-up left constant (ids, weights, offsets, volumes), then waits for
-// the kernel before it (grid_wait).  A wait returns when the whole grid
-// before it has finished and its writes are visible, so the order is the
-// stream's; what overlaps is the launch and the constant loads with the
-// previous kernel's end.  Kernels let the next one start when their blocks
-// exit, the fused stages before their last stores (grid_trigger): started any
-// earlier, its blocks fill the slots that happen to be free and sit unevenly
-// on the SMs (48^3, DW: 218 us per V-cycle when triggered at the start, 160
-// like this, 195 with plain launches, memsets and copies between them).  Data
-// that a kernel of the chain writes is read after the wait, through pointers
-// without __restrict__ (a load from a const __restrict__ pointer may be
-// hoisted above it or go through the read-only path).
+// These launches follow one another as programmatic dependents (launch.cuh):
+// each loads what set-up left constant (ids, weights, offsets, volumes) before
+// it waits for the kernel before it.  Kernels let the next one start when their
+// blocks exit, the fused stages before their last stores (grid_trigger):
+// started any earlier, its blocks fill the slots that happen to be free and sit
+// unevenly on the SMs (48^3, DW: 218 us per V-cycle when triggered at the start,
+// 160 like this, 195 with plain launches, memsets and copies between them).
 //
 // Failure handling: min_dt < 0 and NaN/Inf at level 0 set a sticky device
 // status word; every later kernel sees it and returns, so the run stops at the
@@ -72,6 +66,7 @@
 #include "common.h"
 #include "device_math.cuh"
 #include "dw_math.cuh"
+#include "launch.cuh"
 #include "setup.h"
 #include "solver_internal.h"
 
@@ -98,25 +93,6 @@ void keep_freed_memory(int dev) {
 
 // ---------------------------------------------------------------------------
 // Kernels.
-
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// Launches a kernel that begins with grid_wait as the programmatic dependent
-// of the kernel before it in the stream (`chained`), else in plain stream order.
-template <class... P, class... A>
-void launch(void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t stream, bool chained, A... args) {
-  cudaLaunchConfig_t c = {};
-  cudaLaunchAttribute at;
-  c.gridDim = dim3((unsigned)blocks);
-  c.blockDim = dim3((unsigned)threads);
-  c.stream = stream;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = &at;
-  c.numAttrs = chained ? 1 : 0;
-  cudaLaunchKernelEx(&c, kernel, P(args)...);  // errors: the callers' cudaGetLastError
-}
 
 // The min_dt keys of the level just smoothed: kept as the ones its last step
 // used (for the step factors that a fetch reports), then reset for its next
