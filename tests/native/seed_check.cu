@@ -9,12 +9,13 @@
 namespace {
 
 __global__ void k_check(int64_t n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ r,
-                        double* __restrict__ q, double* __restrict__ s) {
+                        double* __restrict__ q, double* __restrict__ s, double* __restrict__ by) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   r[i] = mgcfd::rcp_fast(b[i]);
   q[i] = mgcfd::div_fast(a[i], b[i]);
   s[i] = mgcfd::sqrt_fast(b[i]);
+  by[i] = mgcfd::div_by(a[i], b[i], mgcfd::rcp_fast(b[i]));
 }
 
 // One row of m terms per thread.
@@ -42,18 +43,19 @@ extern "C" int sum_check(int64_t n, int m, const float* x, double* out) {
   return (int)e;
 }
 
-// Host buffers in (a, b) and out (1/b, a/b, sqrt(b)); returns a cudaError_t value.
-extern "C" int seed_check(int64_t n, const double* a, const double* b, double* r, double* q, double* s) {
+// Host buffers in (a, b) and out (1/b, a/b, sqrt(b), a/b by div_by); returns a cudaError_t value.
+extern "C" int seed_check(int64_t n, const double* a, const double* b, double* r, double* q, double* s, double* by) {
   const size_t bytes = sizeof(double) * (size_t)n;
   double* d = nullptr;
-  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&d), 5 * bytes);
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&d), 6 * bytes);
   if (e) return (int)e;
   if (!(e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice)) &&
       !(e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice))) {
-    k_check<<<(unsigned)((n + 127) / 128), 128>>>(n, d, d + n, d + 2 * n, d + 3 * n, d + 4 * n);
+    k_check<<<(unsigned)((n + 127) / 128), 128>>>(n, d, d + n, d + 2 * n, d + 3 * n, d + 4 * n, d + 5 * n);
     if (!(e = cudaGetLastError()) && !(e = cudaMemcpy(r, d + 2 * n, bytes, cudaMemcpyDeviceToHost)) &&
-        !(e = cudaMemcpy(q, d + 3 * n, bytes, cudaMemcpyDeviceToHost)))
-      e = cudaMemcpy(s, d + 4 * n, bytes, cudaMemcpyDeviceToHost);
+        !(e = cudaMemcpy(q, d + 3 * n, bytes, cudaMemcpyDeviceToHost)) &&
+        !(e = cudaMemcpy(s, d + 4 * n, bytes, cudaMemcpyDeviceToHost)))
+      e = cudaMemcpy(by, d + 5 * n, bytes, cudaMemcpyDeviceToHost);
   }
   cudaFree(d);
   return (int)e;

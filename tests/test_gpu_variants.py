@@ -78,7 +78,7 @@ def native():
 @pytest.fixture(scope="module")
 def seed_check(native):
     def run(a, b):
-        outs = [np.empty(len(b)) for _ in range(3)]
+        outs = [np.empty(len(b)) for _ in range(4)]
         p = [x.ctypes.data_as(C.c_void_p) for x in (a, b, *outs)]
         assert native.seed_check(C.c_int64(len(b)), *p) == 0
         return outs
@@ -92,12 +92,14 @@ def test_seeded_reciprocal_quotient_root(seed_check, kind):
     within 2^-42, so one Newton step leaves 0.5 ulp of rounding and, for the
     root, 2^-42 * 2^-21 * 2^53 = 2^-10 ulp more: 0.5 + 2^-9 is the bound."""
     a, b = _seed_inputs(kind)
-    r, q, s = seed_check(a, b)
+    r, q, s, by = seed_check(a, b)
     A, B = a.astype(np.longdouble), b.astype(np.longdouble)
     slack = 0.5 + 2.0 ** -9
     assert _ulps(r, 1 / B).max() <= slack
     assert _ulps(q, A / B).max() <= slack
     assert _ulps(s, np.sqrt(B)).max() <= slack
+    fast = (b >= 2.0 ** -60) & (b < 2.0 ** 60)
+    np.testing.assert_array_equal(by[fast], (a / b)[fast])  # the set-up's quotients are the host's, bit for bit
 
 
 def test_seeded_forms_keep_the_ieee_special_cases(seed_check):
@@ -107,7 +109,7 @@ def test_seeded_forms_keep_the_ieee_special_cases(seed_check):
     edge = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 2.2e-308, 1.7e308, -1.0, -4.0, 2.0 ** -60,
                      2.0 ** 60, np.nextafter(2.0 ** 60, 0), np.nextafter(2.0 ** -60, 0), 2.0 ** -61, 1e-200, 1e200])
     a, b = (x.ravel().copy() for x in np.meshgrid(edge, edge))
-    r, q, s = seed_check(a, b)
+    r, q, s, by = seed_check(a, b)
     fast_b = (b >= 2.0 ** -60) & (b < 2.0 ** 60)
     fast_q = fast_b & (np.abs(a) >= 2.0 ** -900) & (np.abs(a) < 2.0 ** 900)
     with np.errstate(all="ignore"):
@@ -119,6 +121,9 @@ def test_seeded_forms_keep_the_ieee_special_cases(seed_check):
         ieee = ~nan & ~fast
         assert np.array_equal(got[ieee].view(np.uint64), w[ieee].view(np.uint64))
         assert _ulps(got[fast], ld[fast]).max() <= 0.5 + 2.0 ** -9
+    # (div_by may miss a quotient within 2^-52 ulp of a tie: powers of two by the number below 2^60 are)
+    finite = np.isfinite(a) & ~np.isnan(want[1]) & (b != np.nextafter(2.0 ** 60, 0))
+    assert np.array_equal(by[finite].view(np.uint64), want[1][finite].view(np.uint64))
 
 
 @pytest.mark.parametrize("terms", [1, 2, 6, 7, 14, 40])
