@@ -529,6 +529,205 @@ struct LevelIn {
   int32_t* inv = nullptr;  // input node id -> new node id (global)
 };
 
+// A second stream for the coarse levels of a set-up: it starts behind what the
+// solver's stream holds (uploads and allocations), and the solver's stream
+// waits for it at the join.  An early return waits for it too, before the
+// scratch that its kernels use goes.
+struct SideStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t event = nullptr;
+  int open(cudaStream_t after) {
+    CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+    CK(cudaEventRecord(event, after));
+    CK(cudaStreamWaitEvent(stream, event, 0));
+    return MGCFD_OK;
+  }
+  int join(cudaStream_t into) {
+    if (!stream) return MGCFD_OK;
+    CK(cudaEventRecord(event, stream));
+    CK(cudaStreamWaitEvent(into, event, 0));
+    joined = true;
+    return MGCFD_OK;
+  }
+  ~SideStream() {
+    if (stream && !joined) cudaStreamSynchronize(stream);
+    if (event) cudaEventDestroy(event);
+    if (stream) cudaStreamDestroy(stream);
+  }
+
+ private:
+  bool joined = false;
+};
+
+// The set-up's coarse levels get a stream of their own from this many level-0
+// nodes on.
+constexpr int32_t kSideNodes = 8192;
+
+// One level's tables and state, from its inputs, on stream st with scratch
+// from tmp.
+int build_level(mgcfd_solver* s, cudaStream_t st, Temp& tmp, const Seg& g, const LevelIn& I, int l, int32_t N,
+                int32_t NE, int32_t NB, bool any_computed_volumes, unsigned* fin, int nlevels) {
+  DevLevel& D = s->L[(size_t)l];
+  const int nseg = g.nseg;
+  const bool mixed = s->opt.precision == MGCFD_PRECISION_MIXED;
+  unsigned* err = fin;
+  double* w4all = nullptr;
+  int r;
+  D.n = N; D.ne = NE; D.nb = NB;
+  if ((r = s->alloc(&D.perm, (size_t)N, st)) || (r = s->alloc(&D.vol, (size_t)N, st)) ||
+      (r = s->alloc(&D.inv_vol, (size_t)N, st)) || (r = s->alloc(&D.cbrt_vol, (size_t)N, st)) ||
+      (r = s->alloc(&D.e2n, (size_t)NE, st)) || (r = s->alloc(&D.bidx, (size_t)N, st)) ||
+      (r = s->alloc(&D.bdata, 12 * (size_t)(NB > 0 ? NB : 1), st)))
+    return r;
+  if (mixed) {
+    if ((r = tmp.get(&w4all, 4 * (size_t)NE)) || (r = s->alloc(&D.w4f, (size_t)NE, st)) ||
+        (s->opt.measure_mem_bound && (r = s->alloc(&D.w4, (size_t)NE, st))))
+      return r;
+  } else {
+    if ((r = s->alloc(&D.w4, (size_t)NE, st))) return r;
+    w4all = reinterpret_cast<double*>(D.w4);
+  }
+  if (wants_edge_lists(s, N) && ((r = s->alloc(&D.a_off, (size_t)N + 1, st)) ||
+                                 (r = s->alloc(&D.b_off, (size_t)N + 1, st)) ||
+                                 (r = s->alloc(&D.b_list, (size_t)NE, st))))
+    return r;
+  if (wants_slices(s, N) && (r = s->alloc(&D.sl_off, (size_t)((N + 31) / 32) + 1, st))) return r;
+  if (nseg > 1 && (r = s->alloc(&D.mesh_id, (size_t)N, st))) return r;
+  if (nseg > 1) k_seg_of<<<nblk(N), T, 0, st>>>(N, g.noff, nseg, nullptr, D.mesh_id);
+
+  // Node order: Morton codes within each mesh, its boundary nodes last, then stably by mesh.
+  if (s->opt.renumber == MGCFD_RENUMBER_SPATIAL) {
+    unsigned long long *lo, *hi, *key, *key2;
+    int32_t *val, *val2;
+    if ((r = tmp.get(&lo, 3 * (size_t)nseg)) || (r = tmp.get(&hi, 3 * (size_t)nseg)) ||
+        (r = tmp.get(&key, (size_t)N)) || (r = tmp.get(&key2, (size_t)N)) || (r = tmp.get(&val, (size_t)N)) ||
+        (r = tmp.get(&val2, (size_t)N)))
+      return r;
+    CK(cudaMemsetAsync(lo, 0xff, 24 * (size_t)nseg, st));
+    CK(cudaMemsetAsync(hi, 0, 24 * (size_t)nseg, st));
+    double* box;
+    uint8_t* mark;
+    if ((r = tmp.get(&box, 6 * (size_t)nseg)) || (r = tmp.get(&mark, (size_t)N))) return r;
+    CK(cudaMemsetAsync(mark, 0, (size_t)N, st));
+    if (NB) k_mark_boundary<<<nblk(NB), T, 0, st>>>(NB, g, I.b2n, I.grp, mark);
+    k_bbox<<<nblk(N), T, 0, st>>>(N, I.xyz, g, lo, hi);
+    k_box_scale<<<nblk(3 * (int64_t)nseg), T, 0, st>>>(nseg, lo, hi, box);
+    k_morton<<<nblk(N), T, 0, st>>>(N, I.xyz, g, box, mark, key, val);
+    if (nseg == 1) {
+      if ((r = sort_pairs(tmp, key, key2, val, D.perm, N, 64, st))) return r;
+    } else {
+      int32_t *mkey, *mkey2;
+      if ((r = tmp.get(&mkey, (size_t)N)) || (r = tmp.get(&mkey2, (size_t)N))) return r;
+      if ((r = sort_pairs(tmp, key, key2, val, val2, N, 64, st))) return r;
+      k_seg_of<<<nblk(N), T, 0, st>>>(N, g.noff, nseg, val2, mkey);
+      if ((r = sort_pairs(tmp, mkey, mkey2, val2, D.perm, N, bits_for(nseg - 1), st))) return r;
+    }
+  } else {
+    k_iota<<<nblk(N), T, 0, st>>>(N, D.perm);
+  }
+  k_inverse<<<nblk(N), T, 0, st>>>(N, D.perm, I.inv);
+
+  // Geometry and volumes.
+  double *tv, *wd;
+  int32_t* ge2n;
+  if ((r = tmp.get(&tv, (size_t)NE)) || (r = tmp.get(&wd, 3 * (size_t)NE)) || (r = tmp.get(&ge2n, 2 * (size_t)NE)))
+    return r;
+  if (NE && mixed) k_edge_geometry<true><<<nblk(NE), T, 0, st>>>(NE, g, I.e2n, I.xyz, I.ewt, ge2n, tv, wd, err);
+  else if (NE) k_edge_geometry<false><<<nblk(NE), T, 0, st>>>(NE, g, I.e2n, I.xyz, I.ewt, ge2n, tv, wd, err);
+  if (any_computed_volumes) {
+    int32_t *ikey, *ival, *ikey2, *ival2, *cnt, *off;
+    if ((r = tmp.get(&ikey, 2 * (size_t)NE)) || (r = tmp.get(&ival, 2 * (size_t)NE)) ||
+        (r = tmp.get(&ikey2, 2 * (size_t)NE)) || (r = tmp.get(&ival2, 2 * (size_t)NE)) ||
+        (r = tmp.get(&cnt, (size_t)N + 1)) || (r = tmp.get(&off, (size_t)N + 1)))
+      return r;
+    CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
+    if (NE) k_incidence<<<nblk(NE), T, 0, st>>>(NE, N, ge2n, ikey, ival, cnt);
+    if ((r = sort_pairs(tmp, ikey, ikey2, ival, ival2, 2 * (int64_t)NE, bits_for(N), st))) return r;
+    if ((r = offsets(tmp, cnt, off, N, st))) return r;
+    k_volumes<<<nblk(N), T, 0, st>>>(N, g, off, ival2, tv, I.vol);
+  }
+  k_node_constants<<<nblk(N), T, 0, st>>>(N, D.perm, I.vol, D.vol, D.inv_vol, D.cbrt_vol);
+
+  // Edges: orientation, order, weights, CSR.
+  {
+    unsigned long long *key, *key2;
+    int32_t *val, *order, *acnt, *bcnt;
+    unsigned char* flip;
+    if ((r = tmp.get(&key, (size_t)NE)) || (r = tmp.get(&key2, (size_t)NE)) || (r = tmp.get(&val, (size_t)NE)) ||
+        (r = tmp.get(&order, (size_t)NE)) || (r = tmp.get(&flip, (size_t)NE)) ||
+        (r = tmp.get(&acnt, (size_t)N + 1)) || (r = tmp.get(&bcnt, (size_t)N + 1)))
+      return r;
+    CK(cudaMemsetAsync(acnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
+    CK(cudaMemsetAsync(bcnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
+    if (NE) {
+      const int nb = bits_for(N);
+      k_edge_keys<<<nblk(NE), T, 0, st>>>(NE, nb, ge2n, I.inv, key, val, flip);
+      if ((r = sort_pairs(tmp, key, key2, val, order, NE, 2 * nb, st))) return r;
+      if (mixed) k_edge_finalize<true><<<nblk(NE), T, 0, st>>>(NE, nb, g, key2, order, wd, flip, D.e2n, w4all, acnt, bcnt);
+      else k_edge_finalize<false><<<nblk(NE), T, 0, st>>>(NE, nb, g, key2, order, wd, flip, D.e2n, w4all, acnt, bcnt);
+    }
+    if (wants_edge_lists(s, N)) {
+      int32_t *bkey, *bval, *bkey2;
+      if ((r = tmp.get(&bkey, (size_t)NE)) || (r = tmp.get(&bval, (size_t)NE)) || (r = tmp.get(&bkey2, (size_t)NE)))
+        return r;
+      if ((r = offsets(tmp, acnt, D.a_off, N, st)) || (r = offsets(tmp, bcnt, D.b_off, N, st))) return r;
+      if (NE) {
+        k_b_pairs<<<nblk(NE), T, 0, st>>>(NE, D.e2n, bkey, bval);
+        if ((r = sort_pairs(tmp, bkey, bkey2, bval, D.b_list, NE, bits_for(N), st))) return r;
+      }
+      if (wants_slices(s, N)) {
+        const int32_t ns = (N + 31) / 32;
+        int32_t* width;
+        if ((r = tmp.get(&width, (size_t)ns + 1))) return r;
+        k_slice_width<<<nblk(N), T, 0, st>>>(N, D.a_off, D.b_off, width);
+        if ((r = offsets(tmp, width, D.sl_off, ns, st))) return r;
+        k_copy1<<<1, 1, 0, st>>>(D.sl_off + ns, fin + 1 + nlevels + l);
+      }
+    }
+  }
+
+  // Boundary entries folded per node.
+  {
+    int32_t *key, *val, *key2, *val2, *cnt, *off, *flag, *row;
+    if ((r = tmp.get(&key, (size_t)NB)) || (r = tmp.get(&val, (size_t)NB)) || (r = tmp.get(&key2, (size_t)NB)) ||
+        (r = tmp.get(&val2, (size_t)NB)) || (r = tmp.get(&cnt, (size_t)N + 1)) ||
+        (r = tmp.get(&off, (size_t)N + 1)) || (r = tmp.get(&flag, (size_t)N + 1)) ||
+        (r = tmp.get(&row, (size_t)N + 1)))
+      return r;
+    CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
+    if (NB) {
+      k_bnd_keys<<<nblk(NB), T, 0, st>>>(NB, N, g, I.b2n, I.grp, I.inv, key, val, cnt, err);
+      if ((r = sort_pairs(tmp, key, key2, val, val2, NB, bits_for(N), st))) return r;
+    }
+    if ((r = offsets(tmp, cnt, off, N, st))) return r;
+    CK(cudaMemsetAsync(flag, 0, sizeof(int32_t) * ((size_t)N + 1), st));
+    k_nonempty<<<nblk(N), T, 0, st>>>(N, off, flag);
+    if ((r = offsets(tmp, flag, row, N, st))) return r;
+    k_bnd_fold<<<nblk(N), T, 0, st>>>(N, g, off, val2, I.grp, I.bwt, row, D.bidx, D.bdata);
+    k_copy1<<<1, 1, 0, st>>>(row + N, fin + 1 + l);
+  }
+  if (mixed) {
+    if (NE) k_to_float<<<nblk(4 * (int64_t)NE), T, 0, st>>>(4 * (int64_t)NE, w4all, reinterpret_cast<float*>(D.w4f));
+    if (s->opt.measure_mem_bound) {
+      if (NE) CK(cudaMemcpyAsync(D.w4, w4all, 32 * (size_t)NE, cudaMemcpyDeviceToDevice, st));
+    }
+  }
+  // Per-level state.
+  if ((r = s->alloc(&D.rec, 8 * (size_t)N, st)) || (r = s->alloc(&D.old, 5 * (size_t)N, st)) ||
+      (r = s->alloc(&D.res, 5 * (size_t)N, st)))
+    return r;
+  if (mixed && (r = s->alloc(&D.rec32, 8 * (size_t)N, st))) return r;
+  if (!s->gather) {
+    if ((r = s->alloc(&D.flux, 5 * (size_t)N, st))) return r;
+  } else if (!s->fused) {
+    if (mixed ? (r = s->alloc(&D.fe32, 5 * (size_t)NE, st)) : (r = s->alloc(&D.fe, 5 * (size_t)NE, st))) return r;
+  }
+  if (s->opt.measure_mem_bound && (r = s->alloc(&D.dummy, 5 * (size_t)N, st))) return r;
+  CK(cudaGetLastError());
+  return MGCFD_OK;
+}
+
 }  // namespace
 
 int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
@@ -612,161 +811,21 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
     }
   }
 
+  // Level 0 on the solver's stream, the coarse levels beside it on a second
+  // one: a level's set-up is some fifty short kernels, each a few us of latency
+  // on a coarse level, and the levels do not depend on each other until their
+  // multigrid tables.  (64^3 FP64: 2.03 -> 1.77 ms, 48^3 1.58 -> 1.34.)  On
+  // smaller meshes the host's launches take the time, and one stream is enough.
+  SideStream side;
+  if (nlevels > 1 && total(0, 0) >= kSideNodes && (r = side.open(st))) return r;
+  Temp side_tmp(side.stream ? side.stream : st);
   for (int l = 0; l < nlevels; l++) {
-    DevLevel& D = s->L[(size_t)l];
-    LevelIn& I = in[(size_t)l];
-    const Seg g = seg(l);
-    const int32_t N = total(l, 0), NE = total(l, 1), NB = total(l, 2);
-    D.n = N; D.ne = NE; D.nb = NB;
-    if ((r = s->alloc(&D.perm, (size_t)N)) || (r = s->alloc(&D.vol, (size_t)N)) ||
-        (r = s->alloc(&D.inv_vol, (size_t)N)) || (r = s->alloc(&D.cbrt_vol, (size_t)N)) ||
-        (r = s->alloc(&D.e2n, (size_t)NE)) || (r = s->alloc(&D.bidx, (size_t)N)) ||
-        (r = s->alloc(&D.bdata, 12 * (size_t)(NB > 0 ? NB : 1))))
+    const bool beside = side.stream && l > 0;
+    if ((r = build_level(s, beside ? side.stream : st, beside ? side_tmp : tmp, seg(l), in[(size_t)l], l, total(l, 0),
+                         total(l, 1), total(l, 2), any_computed_volumes, fin, nlevels)))
       return r;
-    double* w4all = nullptr;
-    if (mixed) { if ((r = tmp.get(&w4all, 4 * (size_t)NE))) return r; }
-    else { if ((r = s->alloc(&D.w4, (size_t)NE))) return r; w4all = reinterpret_cast<double*>(D.w4); }
-    const bool lists = wants_edge_lists(s, N);
-    if (lists && ((r = s->alloc(&D.a_off, (size_t)N + 1)) || (r = s->alloc(&D.b_off, (size_t)N + 1)) ||
-                      (r = s->alloc(&D.b_list, (size_t)NE))))
-      return r;
-    if (nseg > 1) {
-      if ((r = s->alloc(&D.mesh_id, (size_t)N))) return r;
-      k_seg_of<<<nblk(N), T, 0, st>>>(N, g.noff, nseg, nullptr, D.mesh_id);
-    }
-
-    // Node order: Morton codes within each mesh, its boundary nodes last, then stably by mesh.
-    if (s->opt.renumber == MGCFD_RENUMBER_SPATIAL) {
-      unsigned long long *lo, *hi, *key, *key2;
-      int32_t *val, *val2;
-      if ((r = tmp.get(&lo, 3 * (size_t)nseg)) || (r = tmp.get(&hi, 3 * (size_t)nseg)) ||
-          (r = tmp.get(&key, (size_t)N)) || (r = tmp.get(&key2, (size_t)N)) || (r = tmp.get(&val, (size_t)N)) ||
-          (r = tmp.get(&val2, (size_t)N)))
-        return r;
-      CK(cudaMemsetAsync(lo, 0xff, 24 * (size_t)nseg, st));
-      CK(cudaMemsetAsync(hi, 0, 24 * (size_t)nseg, st));
-      double* box;
-      uint8_t* mark;
-      if ((r = tmp.get(&box, 6 * (size_t)nseg)) || (r = tmp.get(&mark, (size_t)N))) return r;
-      CK(cudaMemsetAsync(mark, 0, (size_t)N, st));
-      if (NB) k_mark_boundary<<<nblk(NB), T, 0, st>>>(NB, g, I.b2n, I.grp, mark);
-      k_bbox<<<nblk(N), T, 0, st>>>(N, I.xyz, g, lo, hi);
-      k_box_scale<<<nblk(3 * (int64_t)nseg), T, 0, st>>>(nseg, lo, hi, box);
-      k_morton<<<nblk(N), T, 0, st>>>(N, I.xyz, g, box, mark, key, val);
-      if (nseg == 1) {
-        if ((r = sort_pairs(tmp, key, key2, val, D.perm, N, 64, st))) return r;
-      } else {
-        int32_t *mkey, *mkey2;
-        if ((r = tmp.get(&mkey, (size_t)N)) || (r = tmp.get(&mkey2, (size_t)N))) return r;
-        if ((r = sort_pairs(tmp, key, key2, val, val2, N, 64, st))) return r;
-        k_seg_of<<<nblk(N), T, 0, st>>>(N, g.noff, nseg, val2, mkey);
-        if ((r = sort_pairs(tmp, mkey, mkey2, val2, D.perm, N, bits_for(nseg - 1), st))) return r;
-      }
-    } else {
-      k_iota<<<nblk(N), T, 0, st>>>(N, D.perm);
-    }
-    k_inverse<<<nblk(N), T, 0, st>>>(N, D.perm, I.inv);
-
-    // Geometry and volumes.
-    double *tv, *wd;
-    int32_t* ge2n;
-    if ((r = tmp.get(&tv, (size_t)NE)) || (r = tmp.get(&wd, 3 * (size_t)NE)) || (r = tmp.get(&ge2n, 2 * (size_t)NE)))
-      return r;
-    if (NE && mixed) k_edge_geometry<true><<<nblk(NE), T, 0, st>>>(NE, g, I.e2n, I.xyz, I.ewt, ge2n, tv, wd, err);
-    else if (NE) k_edge_geometry<false><<<nblk(NE), T, 0, st>>>(NE, g, I.e2n, I.xyz, I.ewt, ge2n, tv, wd, err);
-    if (any_computed_volumes) {
-      int32_t *ikey, *ival, *ikey2, *ival2, *cnt, *off;
-      if ((r = tmp.get(&ikey, 2 * (size_t)NE)) || (r = tmp.get(&ival, 2 * (size_t)NE)) ||
-          (r = tmp.get(&ikey2, 2 * (size_t)NE)) || (r = tmp.get(&ival2, 2 * (size_t)NE)) ||
-          (r = tmp.get(&cnt, (size_t)N + 1)) || (r = tmp.get(&off, (size_t)N + 1)))
-        return r;
-      CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
-      if (NE) k_incidence<<<nblk(NE), T, 0, st>>>(NE, N, ge2n, ikey, ival, cnt);
-      if ((r = sort_pairs(tmp, ikey, ikey2, ival, ival2, 2 * (int64_t)NE, bits_for(N), st))) return r;
-      if ((r = offsets(tmp, cnt, off, N, st))) return r;
-      k_volumes<<<nblk(N), T, 0, st>>>(N, g, off, ival2, tv, I.vol);
-    }
-    k_node_constants<<<nblk(N), T, 0, st>>>(N, D.perm, I.vol, D.vol, D.inv_vol, D.cbrt_vol);
-
-    // Edges: orientation, order, weights, CSR.
-    {
-      unsigned long long *key, *key2;
-      int32_t *val, *order, *acnt, *bcnt;
-      unsigned char* flip;
-      if ((r = tmp.get(&key, (size_t)NE)) || (r = tmp.get(&key2, (size_t)NE)) || (r = tmp.get(&val, (size_t)NE)) ||
-          (r = tmp.get(&order, (size_t)NE)) || (r = tmp.get(&flip, (size_t)NE)) ||
-          (r = tmp.get(&acnt, (size_t)N + 1)) || (r = tmp.get(&bcnt, (size_t)N + 1)))
-        return r;
-      CK(cudaMemsetAsync(acnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
-      CK(cudaMemsetAsync(bcnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
-      if (NE) {
-        const int nb = bits_for(N);
-        k_edge_keys<<<nblk(NE), T, 0, st>>>(NE, nb, ge2n, I.inv, key, val, flip);
-        if ((r = sort_pairs(tmp, key, key2, val, order, NE, 2 * nb, st))) return r;
-        if (mixed) k_edge_finalize<true><<<nblk(NE), T, 0, st>>>(NE, nb, g, key2, order, wd, flip, D.e2n, w4all, acnt, bcnt);
-        else k_edge_finalize<false><<<nblk(NE), T, 0, st>>>(NE, nb, g, key2, order, wd, flip, D.e2n, w4all, acnt, bcnt);
-      }
-      if (lists) {
-        int32_t *bkey, *bval, *bkey2;
-        if ((r = tmp.get(&bkey, (size_t)NE)) || (r = tmp.get(&bval, (size_t)NE)) || (r = tmp.get(&bkey2, (size_t)NE)))
-          return r;
-        if ((r = offsets(tmp, acnt, D.a_off, N, st)) || (r = offsets(tmp, bcnt, D.b_off, N, st))) return r;
-        if (NE) {
-          k_b_pairs<<<nblk(NE), T, 0, st>>>(NE, D.e2n, bkey, bval);
-          if ((r = sort_pairs(tmp, bkey, bkey2, bval, D.b_list, NE, bits_for(N), st))) return r;
-        }
-        if (wants_slices(s, N)) {
-          const int32_t ns = (N + 31) / 32;
-          int32_t* width;
-          if ((r = tmp.get(&width, (size_t)ns + 1)) || (r = s->alloc(&D.sl_off, (size_t)ns + 1))) return r;
-          k_slice_width<<<nblk(N), T, 0, st>>>(N, D.a_off, D.b_off, width);
-          if ((r = offsets(tmp, width, D.sl_off, ns, st))) return r;
-          k_copy1<<<1, 1, 0, st>>>(D.sl_off + ns, fin + 1 + nlevels + l);
-        }
-      }
-    }
-
-    // Boundary entries folded per node.
-    {
-      int32_t *key, *val, *key2, *val2, *cnt, *off, *flag, *row;
-      if ((r = tmp.get(&key, (size_t)NB)) || (r = tmp.get(&val, (size_t)NB)) || (r = tmp.get(&key2, (size_t)NB)) ||
-          (r = tmp.get(&val2, (size_t)NB)) || (r = tmp.get(&cnt, (size_t)N + 1)) ||
-          (r = tmp.get(&off, (size_t)N + 1)) || (r = tmp.get(&flag, (size_t)N + 1)) ||
-          (r = tmp.get(&row, (size_t)N + 1)))
-        return r;
-      CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)N + 1), st));
-      if (NB) {
-        k_bnd_keys<<<nblk(NB), T, 0, st>>>(NB, N, g, I.b2n, I.grp, I.inv, key, val, cnt, err);
-        if ((r = sort_pairs(tmp, key, key2, val, val2, NB, bits_for(N), st))) return r;
-      }
-      if ((r = offsets(tmp, cnt, off, N, st))) return r;
-      CK(cudaMemsetAsync(flag, 0, sizeof(int32_t) * ((size_t)N + 1), st));
-      k_nonempty<<<nblk(N), T, 0, st>>>(N, off, flag);
-      if ((r = offsets(tmp, flag, row, N, st))) return r;
-      k_bnd_fold<<<nblk(N), T, 0, st>>>(N, g, off, val2, I.grp, I.bwt, row, D.bidx, D.bdata);
-      k_copy1<<<1, 1, 0, st>>>(row + N, fin + 1 + l);
-    }
-    if (mixed) {
-      if ((r = s->alloc(&D.w4f, (size_t)NE))) return r;
-      if (NE) k_to_float<<<nblk(4 * (int64_t)NE), T, 0, st>>>(4 * (int64_t)NE, w4all, reinterpret_cast<float*>(D.w4f));
-      if (s->opt.measure_mem_bound) {
-        if ((r = s->alloc(&D.w4, (size_t)NE))) return r;
-        if (NE) CK(cudaMemcpyAsync(D.w4, w4all, 32 * (size_t)NE, cudaMemcpyDeviceToDevice, st));
-      }
-    }
-    // Per-level state.
-    if ((r = s->alloc(&D.rec, 8 * (size_t)N)) || (r = s->alloc(&D.old, 5 * (size_t)N)) ||
-        (r = s->alloc(&D.res, 5 * (size_t)N)))
-      return r;
-    if (mixed && (r = s->alloc(&D.rec32, 8 * (size_t)N))) return r;
-    if (!s->gather) {
-      if ((r = s->alloc(&D.flux, 5 * (size_t)N))) return r;
-    } else if (!s->fused) {
-      if (mixed ? (r = s->alloc(&D.fe32, 5 * (size_t)NE)) : (r = s->alloc(&D.fe, 5 * (size_t)NE))) return r;
-    }
-    if (s->opt.measure_mem_bound && (r = s->alloc(&D.dummy, 5 * (size_t)N))) return r;
-    CK(cudaGetLastError());
   }
+  if ((r = side.join(st))) return r;
 
   // Multigrid tables.
   for (int l = 0; l + 1 < nlevels; l++) {

@@ -153,11 +153,13 @@ struct mgcfd_solver {
   int32_t stop_max_cycles = 0;
   double stop_drop = 0.0;
 
+  // Device memory of the solver, allocated in the order of `on` (default: the
+  // solver's stream).
   template <class T>
-  int alloc(T** p, size_t count) {
+  int alloc(T** p, size_t count, cudaStream_t on = nullptr) {
     *p = nullptr;
     if (count == 0) return MGCFD_OK;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), count * sizeof(T), stream);
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), count * sizeof(T), on ? on : stream);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return mgcfd::set_error(MGCFD_ERR_NOMEM, "device allocation of " + std::to_string(count * sizeof(T)) +
