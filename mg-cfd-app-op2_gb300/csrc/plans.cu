@@ -365,33 +365,28 @@ __global__ void __launch_bounds__(128) k_plan_flux(int32_t ne, const int2* __res
   const int2 ab = live ? e2n[e] : make_int2(0, 0);
   const int32_t r = live ? eref[e] : 0;
   grid_wait();
-  if (!live) return;
   const bool flip = r < 0;
   const int64_t ce = flip ? (int64_t)~r : (int64_t)r;
   const double wx = ewt[3 * ce], wy = ewt[3 * ce + 1], wz = ewt[3 * ce + 2];
-  double4_32a m = memo[e];
+  double4_32a m = make_double4_32a(0.0, 0.0, 0.0, 0.0);
+  if (live) m = memo[e];
   unsigned long long hx, hy, hz;
   const bool exact = half_bits(wx, flip, &hx) & half_bits(wy, flip, &hy) & half_bits(wz, flip, &hz);
   const bool hit = memo_valid && exact && hx == (unsigned long long)__double_as_longlong(m.x) &&
                    hy == (unsigned long long)__double_as_longlong(m.y) &&
                    hz == (unsigned long long)__double_as_longlong(m.z);
-  if (!hit) {
+  if (live && !hit) {
     const double h = flip ? 0.5 : -0.5;
     const double mag = sqrt(fma(wz, wz, fma(wy, wy, wx * wx)));
     m = make_double4_32a(h * wx, h * wy, h * wz, -(mag * sc) * 0.5);
   }
   const NodePrim a = plan_rec(rec, ab.x);
   const NodePrim b = plan_rec(rec, ab.y);
-  if (!hit) memo[e] = m;
+  if (live && !hit) memo[e] = m;
   double f[5];
   edge_flux(a, b, m.x, m.y, m.z, m.w, f);
-  double* fa = acc + 5 * (int64_t)ab.x;
-  double* fb = acc + 5 * (int64_t)ab.y;
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    atomicAdd(fa + k, f[k]);
-    atomicAdd(fb + k, negate(f[k]));
-  }
+  __shared__ double stage[4][160];
+  add_increments(acc, ab, f, live, stage[threadIdx.x >> 5]);
 }
 
 // The internal increments onto the caller's rows: one thread per (caller

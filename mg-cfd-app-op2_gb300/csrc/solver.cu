@@ -413,7 +413,7 @@ __global__ void k_flux_f64(int32_t ne, const int2* __restrict__ e2n, const doubl
   grid_wait();
   const NodePrim a = load_rec(rec, ab.x);
   const NodePrim b = load_rec(rec, ab.y);
-  if (!live || st->halt) return;
+  if ((GATHER && !live) || st->halt) return;  // (halt: the same for every thread of the launch)
   double f[5];
   edge_flux(a, b, w.x, w.y, w.z, w.w, f);
   if (GATHER) {
@@ -421,13 +421,8 @@ __global__ void k_flux_f64(int32_t ne, const int2* __restrict__ e2n, const doubl
 #pragma unroll
     for (int k = 0; k < 5; k++) o[k] = f[k];
   } else {
-    double* fa = flux + 5 * (int64_t)ab.x;
-    double* fb = flux + 5 * (int64_t)ab.y;
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-      atomicAdd(fa + k, f[k]);
-      atomicAdd(fb + k, negate(f[k]));
-    }
+    extern __shared__ double stage[];
+    add_increments(flux, ab, f, live, stage + 160 * (threadIdx.x >> 5));
   }
 }
 
@@ -1803,7 +1798,8 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
       } else if (mixed) {
         launch(s->gather ? k_flux_mixed<true> : k_flux_mixed<false>, g, et, s->stream, pdl, D.ne, D.e2n, D.w4f, D.rec32, D.flux, D.fe32, s->st);
       } else {
-        launch(s->gather ? k_flux_f64<true> : k_flux_f64<false>, g, et, s->stream, pdl, D.ne, D.e2n, D.w4, D.rec, D.flux, D.fe, s->st);
+        const size_t stage = s->gather ? 0 : 5 * sizeof(double) * (size_t)et;  // add_increments
+        launch_shared(stage, s->gather ? k_flux_f64<true> : k_flux_f64<false>, g, et, s->stream, pdl, D.ne, D.e2n, D.w4, D.rec, D.flux, D.fe, s->st);
       }
       s->launches++;
       if (time_this) {
