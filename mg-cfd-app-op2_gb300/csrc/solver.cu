@@ -634,6 +634,7 @@ __global__ void k_stream(int32_t ne, const int2* __restrict__ e2n, const double4
 struct UpdateArgs {
   int32_t n;
   int32_t level0;
+  int* in_old;          // last stage: cleared once the state is in rec (null: not kept)
   int32_t clear_norms;  // first stage at level 0: the number of norm accumulators to clear, else 0
   double inv_div;       // 1 / (RK + 1 - rk)
   double* rec;
@@ -863,6 +864,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
       return;
     }
   }
+  if (FUSED && LAST && A.in_old && blockIdx.x == 0 && threadIdx.x == 0) *A.in_old = 0;
   // Edge-parallel fused stage: every thread of the block takes part (the
   // barriers are block-wide), whatever its own node's state.
   float ep_hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, ep_lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
@@ -1260,6 +1262,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_stage_small(UpdateArgs A) {
     if (threadIdx.x == 0) { A.st->neg_dt = 1; atomicOr(&A.st->halt, 1); }
     return;
   }
+  if (LAST && A.in_old && blockIdx.x == 0 && threadIdx.x == 0) *A.in_old = 0;
   // The edges, eight at a time; lane v < 5 sums variable v.
   double F = 0.0;
   float hi = 0.0f, lo = 0.0f;
@@ -1390,7 +1393,15 @@ struct BeginArgs {
   double* old;
   const double* cbrt_vol;
   unsigned long long* dt_key;
+  // Plain solvers with the fused stage, which reads the FP64 state of boundary
+  // nodes only and stores every node's in its last stage: the transfer then
+  // leaves the others' state to `old`, where the step begin puts it anyway (64
+  // of the 290 bytes per node of a mixed prolongation), and says so in in_old.
+  const int32_t* bidx;  // null: store every node's state
+  int* in_old;
 };
+
+__device__ __forceinline__ bool stores_state(const BeginArgs& B, int64_t i) { return !B.bidx || B.bidx[i] >= 0; }
 
 // up_pre/up/up_post (mg.h:29-64) as a gather over each coarse node's children,
 // and the coarse level's step begin on the state just written (as in the
@@ -1422,6 +1433,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int
   const int halted = s_halt;  // block-uniform: the block synchronises below
   reset_keys(fine_keys, halted);
   if (halted) return;
+  if (B.in_old && blockIdx.x == 0 && threadIdx.x == 0) *B.in_old = 1;
   const bool live = c < nc && !(seg_stop && seg_stop[mesh_id[c]].halt);  // not a stopped mesh of a batch
   double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sums of squared residuals, one chain per variable
   int bad = 0;
@@ -1446,9 +1458,10 @@ __global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int
       }
       const double avg = rcp_fast((double)(hi - lo));
 #pragma unroll
-      for (int k = 0; k < 5; k++) {
-        x[k] *= avg;
-        if (MIXED || DW) r[k] = x[k];  // (FP64: stored with the primitives)
+      for (int k = 0; k < 5; k++) x[k] *= avg;
+      if ((MIXED || DW) && stores_state(B, c)) {  // (FP64: stored with the primitives)
+#pragma unroll
+        for (int k = 0; k < 5; k++) r[k] = x[k];
       }
     } else {  // no children: state unchanged (avg = 1 on untouched values)
 #pragma unroll
@@ -1481,6 +1494,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_prolong(int32_t nf, const int3
   const int halted = st->halt;  // the same for every thread of the launch
   reset_keys(coarse_keys, halted);
   if (halted) return;
+  if (B.in_old && blockIdx.x == 0 && threadIdx.x == 0) *B.in_old = 1;
   const bool live = i < nf && !(seg_stop && seg_stop[mesh_id[i]].halt);  // not a stopped mesh of a batch
   double x[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   if (live) {
@@ -1495,7 +1509,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_prolong(int32_t nf, const int3
     v.z -= d.y * (cr[2] - fr[2]);
     v.w -= d.z * (cr[3] - fr[3]);
     v4 -= d.w * (cr[4] - fr[4]);
-    if (MIXED || DW) {  // (FP64: stored with the primitives)
+    if ((MIXED || DW) && stores_state(B, i)) {  // (FP64: stored with the primitives)
       r4[0] = v;
       frec[8 * i + 4] = v4;
     }
@@ -1569,10 +1583,16 @@ __global__ void k_cycle_end_seg(int32_t nseg, SegStop* ss, const double* seg_rho
 
 // Fetch helpers: scatter the renumbered rows [off, off + n) back to input
 // order (rows of one mesh, or of the whole level when off = 0).
+// in_old (may be null): non-zero when the rows are in `old` ([.][5]) instead.
 __global__ void k_unpermute(int32_t n, int32_t off, int32_t width, int32_t stride, const double* __restrict__ src,
-                            const int32_t* __restrict__ perm, double* __restrict__ dst) {
+                            const int32_t* __restrict__ perm, double* __restrict__ dst, const int* in_old,
+                            const double* __restrict__ old) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)n * width) return;
+  if (in_old && *in_old) {
+    src = old;
+    stride = 5;
+  }
   const int64_t i = off + t / width, k = t % width;
   dst[(int64_t)(perm[i] - off) * width + k] = src[i * stride + k];
 }
@@ -1704,30 +1724,43 @@ unsigned long long* level_key_used(mgcfd_solver* s, int level) {
 
 template <bool M, bool S, bool W>
 void launch_prolong(const DevLevel& F, const DevLevel& Cl, const DevStatus* st, const SegStop* ss,
-                    unsigned long long* key, const KeyReset& coarse_keys, cudaStream_t stream, bool chained) {
-  const BeginArgs b{F.rec2, F.rec32, F.old, F.cbrt_vol, key};
+                    unsigned long long* key, const KeyReset& coarse_keys, int* in_old, cudaStream_t stream,
+                    bool chained) {
+  const BeginArgs b{F.rec2, F.rec32, F.old, F.cbrt_vol, key, in_old ? F.bidx : nullptr, in_old};
   launch(k_prolong<M, S, W>, grid(F.n, kNodeThreads), kNodeThreads, stream, chained, F.n, F.n2mg, F.dvec, F.rec,
          F.res, Cl.res, st, F.mesh_id, ss, b, coarse_keys);
 }
 using ProlongFn = void (*)(const DevLevel&, const DevLevel&, const DevStatus*, const SegStop*, unsigned long long*,
-                           const KeyReset&, cudaStream_t, bool);
+                           const KeyReset&, int*, cudaStream_t, bool);
 // Indexed by precision (FP64, MIXED, DW) * 2 + seg.
 const ProlongFn kProlong[6] = {launch_prolong<0, 0, 0>, launch_prolong<0, 1, 0>, launch_prolong<1, 0, 0>,
                                launch_prolong<1, 1, 0>, launch_prolong<0, 0, 1>, launch_prolong<0, 1, 1>};
 
 template <bool N, bool M, bool S, bool W>
 void launch_restrict(const DevLevel& F, const DevLevel& Cl, DevStatus* st, const SegStop* ss, unsigned long long* key,
-                     const KeyReset& fine_keys, cudaStream_t stream, bool chained) {
-  const BeginArgs b{Cl.rec2, Cl.rec32, Cl.old, Cl.cbrt_vol, key};
+                     const KeyReset& fine_keys, int* in_old, cudaStream_t stream, bool chained) {
+  const BeginArgs b{Cl.rec2, Cl.rec32, Cl.old, Cl.cbrt_vol, key, in_old ? Cl.bidx : nullptr, in_old};
   launch(k_restrict<N, M, S, W>, grid(Cl.n, kNodeThreads), kNodeThreads, stream, chained, Cl.n, Cl.ch_off, Cl.ch_list,
          F.rec, Cl.rec, F.res, st, Cl.mesh_id, ss, b, fine_keys);
 }
 using RestrictFn = void (*)(const DevLevel&, const DevLevel&, DevStatus*, const SegStop*, unsigned long long*,
-                            const KeyReset&, cudaStream_t, bool);
+                            const KeyReset&, int*, cudaStream_t, bool);
 const RestrictFn kRestrict[6] = {launch_restrict<0, 0, 0, 0>, launch_restrict<0, 0, 1, 0>, launch_restrict<0, 1, 0, 0>,
                                  launch_restrict<0, 1, 1, 0>, launch_restrict<0, 0, 0, 1>, launch_restrict<0, 0, 1, 1>};
 // With the level-0 norms: plain solvers with the fused stage, MIXED and DW.
 const RestrictFn kRestrictNorms[2] = {launch_restrict<1, 1, 0, 0>, launch_restrict<1, 0, 0, 1>};
+
+// Where a level's transfers and stages note that its state is in `old` (null:
+// the transfers store it into rec).  Not in batches, whose stopped meshes take
+// no further stages, nor beside the -b probe, which reads rec; and only on
+// levels whose records (64 bytes a node) do not stay in the L2, where the bytes
+// are saved and not just a store: 200^3 mixed V-cycle 2.94 -> 2.88 ms, pair sums
+// 2.60 -> 2.54, 100^3 equal, 48^3 115 -> 118 us for the look at bidx.
+constexpr int32_t kStateInOldNodes = 1 << 19;
+int* state_in_old(mgcfd_solver* s, int level) {
+  const bool on = s->fused && s->nseg == 1 && !s->opt.measure_mem_bound && s->L[(size_t)level].n >= kStateInOldNodes;
+  return on ? &s->st->in_old[level] : nullptr;
+}
 
 KeyReset key_reset(mgcfd_solver* s, int level) {
   return KeyReset{level_key(s, level), level_key_used(s, level), s->nseg};
@@ -1810,6 +1843,7 @@ int enqueue_smooth(mgcfd_solver* s, int level) {
     UpdateArgs A;
     A.n = D.n; A.level0 = level == 0 && !norms_in_restrict(s); A.inv_div = 1.0 / (double)(kRK + 1 - rk);
     A.clear_norms = level == 0 && rk == 0 ? s->nseg : 0;
+    A.in_old = last ? state_in_old(s, level) : nullptr;
     A.rec = D.rec; A.rec2 = D.rec2; A.rec32 = D.rec32; A.old = D.old; A.flux = D.flux; A.fe = D.fe; A.fe32 = D.fe32;
     A.a_off = D.a_off; A.b_off = D.b_off; A.b_list = D.b_list; A.inv_vol = D.inv_vol; A.bidx = D.bidx;
     A.bdata = D.bdata; A.res = D.res; A.dt_key = key; A.st = s->st;
@@ -1901,7 +1935,8 @@ int enqueue_iteration(mgcfd_solver* s) {
     const int p = precision_index(s);
     const RestrictFn fn = s->level == 1 && norms_in_restrict(s) ? kRestrictNorms[p - 1]
                                                                 : kRestrict[2 * p + (s->nseg > 1 ? 1 : 0)];
-    fn(F, Cl, s->st, ss, level_key(s, s->level), key_reset(s, s->level - 1), s->stream, chained(s));
+    fn(F, Cl, s->st, ss, level_key(s, s->level), key_reset(s, s->level - 1), state_in_old(s, s->level), s->stream,
+       chained(s));
     s->begun = true;
     s->launches++;
     if (s->level == levels - 1) s->up = false;
@@ -1912,7 +1947,7 @@ int enqueue_iteration(mgcfd_solver* s) {
     // The fine level's next smoothing step begins in the prolongation.
     kProlong[2 * precision_index(s) + (s->nseg > 1 ? 1 : 0)](F, Cl, s->st, s->nseg > 1 ? s->seg_stop : nullptr,
                                                                    level_key(s, s->level), key_reset(s, s->level + 1),
-                                                                   s->stream, chained(s));
+                                                                   state_in_old(s, s->level), s->stream, chained(s));
     s->begun = true;
     s->launches++;
     if (s->level == 0) {
@@ -2481,21 +2516,22 @@ int fetch_rows(mgcfd_solver* s, int32_t level, int32_t q, int32_t off, int32_t n
   const unsigned long long* keys = level_key_used(s, level);
   switch (q) {
     case MGCFD_Q_VARIABLES:
-      k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 8, D.rec, D.perm, s->fetch_buf);
+      k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 8, D.rec, D.perm, s->fetch_buf,
+                                                               state_in_old(s, level), D.old);
       break;
     case MGCFD_Q_FLUXES:
-      if (D.flux) k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 5, D.flux, D.perm, s->fetch_buf);
+      if (D.flux) k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 5, D.flux, D.perm, s->fetch_buf, nullptr, nullptr);
       else CK(cudaMemsetAsync(s->fetch_buf, 0, sizeof(double) * 5 * (size_t)n, s->stream));
       break;
     case MGCFD_Q_RESIDUALS:
-      k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 5, D.res, D.perm, s->fetch_buf);
+      k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 5, D.res, D.perm, s->fetch_buf, nullptr, nullptr);
       break;
     case MGCFD_Q_OLD_VARIABLES:
-      k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 5, D.old, D.perm, s->fetch_buf);
+      k_unpermute<<<grid((int64_t)n * 5, T), T, 0, s->stream>>>(n, off, 5, 5, D.old, D.perm, s->fetch_buf, nullptr, nullptr);
       break;
     case MGCFD_Q_VOLUMES:
       width = 1;
-      k_unpermute<<<grid(n, T), T, 0, s->stream>>>(n, off, 1, 1, D.vol, D.perm, s->fetch_buf);
+      k_unpermute<<<grid(n, T), T, 0, s->stream>>>(n, off, 1, 1, D.vol, D.perm, s->fetch_buf, nullptr, nullptr);
       break;
     case MGCFD_Q_STEP_FACTORS:
       width = 1;

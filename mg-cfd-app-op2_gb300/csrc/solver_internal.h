@@ -38,6 +38,11 @@ struct DevStatus {
   int pad;
   double rho_first;
   double rho_last;
+  // Plain solvers with the fused stage: non-zero while a level's state is in
+  // `old` only (a transfer has begun its step), zero once its last stage has
+  // stored it into rec.  Set by the kernels that do so, so it holds wherever
+  // a solve stopped.
+  int in_old[kMaxLevels];
 };
 
 // Per-mesh stop rule of a batched solver (the serving loop's cohorts): like

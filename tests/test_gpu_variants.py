@@ -216,3 +216,25 @@ def test_small_levels_equal_the_other_stage(kind, form):
         else:
             np.testing.assert_array_equal(got[l], want[l])
     np.testing.assert_allclose(norms, wnorms, rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("n", [8, 30, 81])  # small levels throughout or below; a level 0 that keeps its begun state in one array
+@pytest.mark.parametrize("form", ["mixed", "dw"])
+def test_states_between_steps(n, form):
+    """Every level's variables after every smoothing step and its transfer (the
+    fused stage leaves a begun level's state in one array and a finished one's in
+    another), against the gather increment: bit for bit in mixed precision; DW's
+    gather sums in another form, within the pairs' 2^-42 of each variable's scale."""
+    mesh = mgcfd.HostMesh.generate(n, 3, 5)
+    a = mgcfd.Solver(mesh, 0.6, 2.0, precision=form)
+    b = mgcfd.Solver(mesh, 0.6, 2.0, precision=form, increment="gather")
+    for _ in range(9):  # two V-cycles of four steps and one step more
+        assert a.step() == b.step()
+        for l in range(3):
+            x, y = a.fetch(l), b.fetch(l)
+            if form == "mixed":
+                np.testing.assert_array_equal(x, y)
+            else:
+                np.testing.assert_allclose(x, y, rtol=0, atol=2.0 ** -42 * np.abs(y).max())
+    a.close()
+    b.close()
