@@ -749,7 +749,9 @@ __device__ __forceinline__ void block_norms(double* srms, double* srho, int* sba
 // stage with pair sums is latency-bound: capped at 48 registers (10 blocks
 // per SM, a few bytes spilled) it runs 2% faster; the DW stage capped at 64
 // (8 blocks, no spill) 1.5% faster than at its own 72, and slower at 56
-// (spills).  Every other form keeps the
+// (spills); the last mixed stage over sliced lists capped at 56 (9 blocks; it
+// takes 63) 2% of the V-cycle faster (200^3 2.88 -> 2.81 ms, 100^3 503 -> 495 us),
+// and slower on small levels when capped further.  Every other form keeps the
 // compiler's own register choice: a minimum of 0 blocks is no constraint,
 // whereas a minimum of 1 lets it grow to 70-80 registers and lose occupancy.
 // Fused stage, STAGE (option stage_neighbour_ids): the block's neighbour ids
@@ -786,7 +788,7 @@ constexpr int kEpChunk = 768;
 // DW: the state goes to rec and the next stage's primitives to rec2 as pairs.
 template <bool GATHER, bool LAST, bool MIXED, bool SEG, bool PAIR = false, bool FUSED = false, int FV = 0,
           bool DW = false>
-__global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED && DW) ? 8 : 0) k_update(UpdateArgs A) {
+__global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED && DW) ? 8 : (FUSED && MIXED && LAST && FV == 3) ? 9 : 0) k_update(UpdateArgs A) {
   constexpr bool STAGE = FV == 1;  // neighbour ids staged by cp.async
   constexpr bool EP = FV == 2;     // edge-parallel ends through shared memory
   constexpr bool SLICED = FV == 3;  // sliced edge lists
