@@ -75,6 +75,9 @@ using namespace mgcfd;
 namespace {
 
 constexpr int kNodeThreads = 128;
+// Small levels: threads per node, and nodes per block (half a slice).
+constexpr int kSmallLanes = 8;
+constexpr int kSmallNodes = kNodeThreads / kSmallLanes;
 
 // Keep freed solver and setup memory in the device's default pool, so that
 // repeated solves (batches, serving) do not map fresh memory from the
@@ -1181,8 +1184,6 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
 // runs k_update).  FP64 replaces the atomics by sums in a fixed order and the
 // edge's flux is computed at both ends.
 // P: 0 FP64, 1 MIXED, 2 DW.
-constexpr int kSmallLanes = 8;
-constexpr int kSmallNodes = kNodeThreads / kSmallLanes;  // nodes per block: half a slice
 
 struct DwTerm {  // one product (or value) of a double-word sum, as acc_add_prod adds it
   float p, e;
@@ -1475,6 +1476,78 @@ __global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int
   block_norms(srms, srho, sbad, ((q[0] + q[1]) + (q[2] + q[3])) + q[4], q[0], bad, st);
 }
 
+// The same with eight threads per coarse node, for small coarse levels of plain
+// solvers: each of a node's lanes loads one child, and lane v adds variable v
+// over the children in list order -- k_restrict's sums, bit for bit, without its
+// eight dependent rounds of loads.
+template <bool NORMS, bool MIXED, bool DW>
+__global__ void __launch_bounds__(kNodeThreads) k_restrict_small(int32_t nc, const int32_t* __restrict__ ch_off,
+                                                                 const int32_t* __restrict__ ch_list,
+                                                                 const double* frec, double* crec, const double* fres,
+                                                                 DevStatus* st, BeginArgs B, KeyReset fine_keys) {
+  __shared__ double s_x[kSmallNodes][kSmallLanes][5];
+  __shared__ double srms[NORMS ? kNodeThreads : 1], srho[NORMS ? kNodeThreads : 1];
+  __shared__ int sbad[NORMS ? kNodeThreads : 1];
+  __shared__ int s_halt;
+  const int u = threadIdx.x / kSmallLanes, l = threadIdx.x % kSmallLanes;
+  const int64_t c = (int64_t)blockIdx.x * kSmallNodes + u;
+  const bool in = c < nc;
+  const int32_t lo = in ? ch_off[c] : 0, count = in ? ch_off[c + 1] - lo : 0;
+  const int32_t most = __reduce_max_sync(0xffffffffu, count);
+  int64_t f = l < count ? ch_list[lo + l] : -1;
+  grid_wait();
+  if (threadIdx.x == 0) s_halt = st->halt;
+  double row[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, r2 = 0.0, rr = 0.0, x = 0.0;
+  int bad = 0;
+  auto load_child = [&] {
+    if (f < 0) return;
+    const double4_32a v = *reinterpret_cast<const double4_32a*>(frec + 8 * f);
+    row[0] = v.x; row[1] = v.y; row[2] = v.z; row[3] = v.w; row[4] = frec[8 * f + 4];
+    if (NORMS) {
+      const double* d = fres + 5 * f;
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        r2 += d[k] * d[k];
+        bad += not_finite(row[k]) ? 1 : 0;
+      }
+      rr += d[0] * d[0];
+    }
+  };
+  load_child();
+  __syncthreads();
+  const int halted = s_halt;  // block-uniform: the block synchronises below
+  reset_keys(fine_keys, halted);
+  if (halted) return;
+  if (B.in_old && blockIdx.x == 0 && threadIdx.x == 0) *B.in_old = 1;
+  for (int32_t j0 = 0; j0 < most; j0 += kSmallLanes) {
+    if (j0 > 0) {
+      f = j0 + l < count ? ch_list[lo + j0 + l] : -1;
+      load_child();
+      __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < 5; k++) s_x[u][l][k] = row[k];
+    __syncwarp();
+    if (l < 5)
+      for (int e = 0; e < kSmallLanes && j0 + e < count; e++) x += s_x[u][e][l];
+  }
+  if (in && l < 5) {
+    if (count > 0) {
+      x *= rcp_fast((double)count);
+      if ((MIXED || DW) && stores_state(B, c)) crec[8 * c + l] = x;  // (FP64: stored with the primitives)
+    } else {  // no children: state unchanged (avg = 1 on untouched values)
+      x = crec[8 * c + l];
+    }
+  }
+  double state[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) state[k] = __shfl_sync(0xffffffffu, x, k, kSmallLanes);
+  step_begin_core<MIXED, false, DW>(c, in && l == 0, state, crec, B.rec2, B.rec32, B.old, B.cbrt_vol, B.dt_key,
+                                    nullptr);
+  if (!NORMS) return;
+  block_norms(srms, srho, sbad, r2, rr, bad, st);
+}
+
 // down_kernel (mg.h:66-88) with the parent offsets precomputed.  The fine
 // level's next smoothing step begins here (step_begin_core on the new state
 // while it is in registers) instead of in a separate pass that reads the
@@ -1752,6 +1825,23 @@ const RestrictFn kRestrict[6] = {launch_restrict<0, 0, 0, 0>, launch_restrict<0,
 // With the level-0 norms: plain solvers with the fused stage, MIXED and DW.
 const RestrictFn kRestrictNorms[2] = {launch_restrict<1, 1, 0, 0>, launch_restrict<1, 0, 0, 1>};
 
+template <bool N, bool M, bool W>
+void launch_restrict_small(const DevLevel& F, const DevLevel& Cl, DevStatus* st, const SegStop*,
+                           unsigned long long* key, const KeyReset& fine_keys, int* in_old, cudaStream_t stream,
+                           bool chained) {
+  const BeginArgs b{Cl.rec2, Cl.rec32, Cl.old, Cl.cbrt_vol, key, in_old ? Cl.bidx : nullptr, in_old};
+  launch(k_restrict_small<N, M, W>, grid(Cl.n, kSmallNodes), kNodeThreads, stream, chained, Cl.n, Cl.ch_off,
+         Cl.ch_list, F.rec, Cl.rec, F.res, st, b, fine_keys);
+}
+// Indexed by precision (FP64, MIXED, DW) * 2 + norms (MIXED and DW only).
+const RestrictFn kRestrictSmall[6] = {launch_restrict_small<0, 0, 0>, nullptr,
+                                      launch_restrict_small<0, 1, 0>, launch_restrict_small<1, 1, 0>,
+                                      launch_restrict_small<0, 0, 1>, launch_restrict_small<1, 0, 1>};
+// The largest coarse level they restrict to.  V-cycle without / with, us: 8^3
+// FP64 73.7 / 67.6, mixed 71.7 / 63.5; 32^3 mixed 90.1 / 81.2; 64^3 (32^3 coarse
+// nodes, past the line) FP64 with the line at 16K 359.7, at 64K 369.1.
+constexpr int32_t kRestrictSmallNodes = 16384;
+
 // Where a level's transfers and stages note that its state is in `old` (null:
 // the transfers store it into rec).  Not in batches, whose stopped meshes take
 // no further stages, nor beside the -b probe, which reads rec; and only on
@@ -1935,8 +2025,10 @@ int enqueue_iteration(mgcfd_solver* s) {
     // The coarse level's smoothing step begins in the restriction, which also
     // takes the level-0 norms of the step just smoothed where that left them.
     const int p = precision_index(s);
-    const RestrictFn fn = s->level == 1 && norms_in_restrict(s) ? kRestrictNorms[p - 1]
-                                                                : kRestrict[2 * p + (s->nseg > 1 ? 1 : 0)];
+    const bool norms = s->level == 1 && norms_in_restrict(s);
+    const RestrictFn fn = s->nseg == 1 && Cl.n <= kRestrictSmallNodes ? kRestrictSmall[2 * p + (norms ? 1 : 0)]
+                          : norms                                     ? kRestrictNorms[p - 1]
+                                                                      : kRestrict[2 * p + (s->nseg > 1 ? 1 : 0)];
     fn(F, Cl, s->st, ss, level_key(s, s->level), key_reset(s, s->level - 1), state_in_old(s, s->level), s->stream,
        chained(s));
     s->begun = true;

@@ -238,3 +238,21 @@ def test_states_between_steps(n, form):
                 np.testing.assert_allclose(x, y, rtol=0, atol=2.0 ** -42 * np.abs(y).max())
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("form", ["mixed", "dw"])
+def test_small_restriction_equals_the_other(form):
+    """Restriction with eight threads per coarse node (plain solvers) against a
+    batch's, bit for bit: random maps with up to a dozen and more children per
+    coarse node (two rounds), coarse nodes without any, and the level-0 norms."""
+    levels = irregular_levels(4000, 3, 21)
+    solo = mgcfd.Solver(levels, 0.5, 1.0, precision=form)
+    pair = mgcfd.Batch([levels, levels], [0.5, 0.5], [1.0, 1.0], precision=form)
+    for s in (solo, pair):
+        s.run(2)
+        assert s.synchronize() == 0
+    for l in range(3):
+        np.testing.assert_array_equal(solo.fetch(l), pair.fetch_mesh(0, l))
+    np.testing.assert_allclose(solo.norms()[1:], pair.mesh_status(0)[1:], rtol=1e-6, atol=0)
+    solo.close()
+    pair.close()
