@@ -67,7 +67,10 @@ def algorithmic_flux_bytes(nnodes: int, nedges: int, precision: str = "fp64", in
     words (32 B); per node the primitives read (64 B), old state (40 B), 1/vol,
     boundary index and table offset (16 B), then the next primitives written
     (64 B) in the first two stages and the state and residual (80 B) in the
-    last: 184 and 200 B, 568/3 B per node on average."""
+    last: 184 and 200 B, 568/3 B per node on average.
+    (The fused models count each edge's lists as CSR arrays would hold them.  The
+    sliced lists the stages read store both ends' weights, 40 B per edge in mixed
+    precision and 72 B for DW.)"""
     if precision == "dw" and increment == "fused":
         return 48 * nedges + (568 * nnodes) // 3
     if precision == "dw":

@@ -337,7 +337,9 @@ enum {
 typedef struct mgcfd_solver_options {
   int32_t precision;         /* MGCFD_PRECISION_*                                   */
   int32_t increment;         /* MGCFD_INCREMENT_*; AUTO = ATOMIC for FP64 and FUSED
-                                for MIXED (the fastest of each on GB300)           */
+                                for MIXED and DW (the fastest of each on GB300).
+                                Plain FP64 solvers of up to 32768 nodes sum their
+                                levels up to 4096 nodes in a fixed order instead   */
   int32_t renumber;          /* MGCFD_RENUMBER_*                                    */
   int32_t use_graph;         /* capture one V-cycle as a CUDA graph and replay it  */
   int32_t measure_mem_bound; /* also run unstructured_stream each RK stage (-b)   */
