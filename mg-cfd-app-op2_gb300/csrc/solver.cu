@@ -735,14 +735,23 @@ __device__ __forceinline__ bool block_sums(double* srms, double* srho, int* sbad
 }
 
 // ... added to a plain solver's norms with one atomic per sum.  A NaN or
-// infinity stops the solver (euler3d.cpp:539-548).
+// infinity stops the solver (euler3d.cpp:539-548): `halt` is the bit to set.
 __device__ __forceinline__ void block_norms(double* srms, double* srho, int* sbad, double r2, double rr, int bad,
-                                            DevStatus* st) {
+                                            DevStatus* st, int halt) {
   if (block_sums(srms, srho, sbad, r2, rr, bad)) {
     atomicAdd(&st->rms_acc, r2);
     atomicAdd(&st->rho_acc, rr);
-    if (bad) { atomicAdd(&st->bad_count, bad); atomicOr(&st->halt, 1); }
+    if (bad) { atomicAdd(&st->bad_count, bad); atomicOr(&st->halt, halt); }
   }
+}
+
+// What a stage does on finding `halt` set.  A restriction that finds bad
+// values ends its own launch (kHaltAfter): half a level restricted would leave
+// the other half's state in whichever of rec and `old` does not hold it.  The
+// stage after it makes the stop final, so that no later restriction takes the
+// bit for its own.
+__device__ __forceinline__ void settle_halt(int halt, DevStatus* st) {
+  if (halt == kHaltAfter && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&st->halt, kHalt);
 }
 
 // compute_bnd_node_flux_kernel + time_step_kernel (+ residual_kernel,
@@ -856,7 +865,10 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   }
   if (STAGE) cp_async_wait_all();
   __syncthreads();
-  if (s_halt) return;  // block-uniform: the reduction below synchronises
+  if (s_halt) {  // block-uniform: the reduction below synchronises
+    settle_halt(s_halt, A.st);
+    return;
+  }
   int32_t mid = 0;
   double min_dt;
   if (SEG) {
@@ -865,7 +877,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
   } else {
     min_dt = dkey_inv(*A.dt_key);
     if (min_dt < 0.0) {  // euler3d.cpp:480: abort before the step factor is used
-      if (threadIdx.x == 0) { A.st->neg_dt = 1; atomicOr(&A.st->halt, 1); }
+      if (threadIdx.x == 0) { A.st->neg_dt = 1; atomicOr(&A.st->halt, kHalt); }
       return;
     }
   }
@@ -1169,7 +1181,7 @@ __global__ void __launch_bounds__(kNodeThreads, (FUSED && PAIR) ? 10 : (FUSED &&
     if (sbad[t]) atomicAdd(A.seg_bad + m0 + t, sbad[t]);
     return;
   }
-  block_norms(srms, srho, sbad, r2, rr, bad, A.st);
+  block_norms(srms, srho, sbad, r2, rr, bad, A.st, kHalt);
 }
 
 // One RK stage of a small level, eight threads per node (plain solvers).
@@ -1260,9 +1272,12 @@ __global__ void __launch_bounds__(kNodeThreads) k_stage_small(UpdateArgs A) {
     if (l < 5) old = A.old[5 * i + l];
   }
   __syncthreads();
-  if (s_halt) return;  // block-uniform: the reduction below synchronises
+  if (s_halt) {  // block-uniform: the reduction below synchronises
+    settle_halt(s_halt, A.st);
+    return;
+  }
   if (min_dt < 0.0) {  // euler3d.cpp:480: abort before the step factor is used
-    if (threadIdx.x == 0) { A.st->neg_dt = 1; atomicOr(&A.st->halt, 1); }
+    if (threadIdx.x == 0) { A.st->neg_dt = 1; atomicOr(&A.st->halt, kHalt); }
     return;
   }
   if (LAST && A.in_old && blockIdx.x == 0 && threadIdx.x == 0) *A.in_old = 0;
@@ -1385,7 +1400,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_stage_small(UpdateArgs A) {
     }
   }
   if (!LAST || !A.level0) return;
-  block_norms(srms, srho, sbad, r2, rr, bad, A.st);
+  block_norms(srms, srho, sbad, r2, rr, bad, A.st, kHalt);
 }
 
 // The step-begin arrays of the level that a transfer writes, whose next
@@ -1433,7 +1448,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int
   grid_wait();
   if (threadIdx.x == 0) s_halt = st->halt;
   __syncthreads();
-  const int halted = s_halt;  // block-uniform: the block synchronises below
+  const int halted = NORMS ? s_halt & kHalt : s_halt;  // block-uniform: the block synchronises below
   reset_keys(fine_keys, halted);
   if (halted) return;
   if (B.in_old && blockIdx.x == 0 && threadIdx.x == 0) *B.in_old = 1;
@@ -1473,7 +1488,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_restrict(int32_t nc, const int
   }
   step_begin_core<MIXED, SEG, DW>(c, live, x, crec, B.rec2, B.rec32, B.old, B.cbrt_vol, B.dt_key, mesh_id);
   if (!NORMS) return;
-  block_norms(srms, srho, sbad, ((q[0] + q[1]) + (q[2] + q[3])) + q[4], q[0], bad, st);
+  block_norms(srms, srho, sbad, ((q[0] + q[1]) + (q[2] + q[3])) + q[4], q[0], bad, st, kHaltAfter);
 }
 
 // The same with eight threads per coarse node, for small coarse levels of plain
@@ -1515,7 +1530,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_restrict_small(int32_t nc, con
   };
   load_child();
   __syncthreads();
-  const int halted = s_halt;  // block-uniform: the block synchronises below
+  const int halted = NORMS ? s_halt & kHalt : s_halt;  // block-uniform: the block synchronises below
   reset_keys(fine_keys, halted);
   if (halted) return;
   if (B.in_old && blockIdx.x == 0 && threadIdx.x == 0) *B.in_old = 1;
@@ -1545,7 +1560,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_restrict_small(int32_t nc, con
   step_begin_core<MIXED, false, DW>(c, in && l == 0, state, crec, B.rec2, B.rec32, B.old, B.cbrt_vol, B.dt_key,
                                     nullptr);
   if (!NORMS) return;
-  block_norms(srms, srho, sbad, r2, rr, bad, st);
+  block_norms(srms, srho, sbad, r2, rr, bad, st, kHaltAfter);
 }
 
 // down_kernel (mg.h:66-88) with the parent offsets precomputed.  The fine
@@ -1631,7 +1646,7 @@ __global__ void k_cycle_end(DevStatus* st, double n0, int32_t max_cycles, double
   st->rho_last = rho;
   if (c >= max_cycles || (drop > 0.0 && c > 1 && rho <= drop * st->rho_first)) {
     st->stopped = 1;
-    st->halt = 1;
+    st->halt = kHalt;
   }
 }
 

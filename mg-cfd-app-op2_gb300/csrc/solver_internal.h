@@ -22,11 +22,15 @@ constexpr int kMaxDevices = 64;
     if (e_ != cudaSuccess) return mgcfd::set_error(MGCFD_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Bits of DevStatus::halt.
+constexpr int kHalt = 1;       // no kernel does any more work
+constexpr int kHaltAfter = 2;  // ... from the kernel after the restriction that set it on
+
 struct DevStatus {
   unsigned long long dt_key[kMaxLevels];  // order-preserving key of each level's min_dt (the step
                                            // begun last: a transfer begins the next step of the level it writes)
   unsigned long long dt_key_used[kMaxLevels];  // the key each level's last finished step used
-  int halt;                                // non-zero: stop all further work
+  int halt;                                // kHalt, kHaltAfter: stop all further work
   int neg_dt;                              // min_dt < 0 seen
   int bad_count;                           // NaN/Inf count at level 0
   int stopped;                             // the stop rule ended the solve (not an error)
