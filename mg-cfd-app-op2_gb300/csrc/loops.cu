@@ -44,13 +44,6 @@ int grid_reduce(int64_t n) {
 }
 
 // A kernel that begins with grid_wait, behind the one before it on the stream.
-// A smoothing step begins (get_min_dt) and a level-0 step ends (calc_rms,
-// count_bad_vals) with a launch in plain order: after a run whose launches were
-// programmatic dependents throughout, every later set-up of a solver in the
-// process took 130-190 us longer for each stream that had carried one (set-up
-// of 18x14x10, 3 levels, after twelve such streams: 3.1 ms against 0.94; now
-// 1.0).  Three per-loop V-cycles at 100^3 take 4.91 ms for it, 4.86 without the
-// plain launches and 5.62 with all of them plain.
 template <class... P, class... A>
 void chain(void (*kernel)(P...), int blocks, void* stream, A... args) {
   launch(kernel, blocks, kThreads, static_cast<cudaStream_t>(stream), true, args...);
@@ -459,7 +452,7 @@ extern "C" int mgcfd_op_get_min_dt(int32_t n, const double* dt, double* min_dt, 
   CHECK_N(n, "mgcfd_op_get_min_dt");
   CHECK_PTR(dt, n, "get_min_dt");
   if (!min_dt) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_get_min_dt: null output");
-  launch(k_set_scalar, 1, 1, STREAM(s), false, min_dt, DBL_MAX);
+  launch(k_set_scalar, 1, 1, STREAM(s), true, min_dt, DBL_MAX);
   if (n > 0) chain(k_min_dt, grid_reduce(n), s, n, dt, min_dt);
   return launch_status("get_min_dt");
 }
@@ -546,7 +539,7 @@ extern "C" int mgcfd_op_calc_rms(int32_t n, const double* res, double* rms, void
   CHECK_PTR(res, n, "calc_rms");
   if (!rms) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_calc_rms: null output");
   if (n == 0) return MGCFD_OK;
-  launch(k_sum_squares, grid_reduce(5 * (int64_t)n), kThreads, STREAM(s), false, 5 * (int64_t)n, res, rms);
+  chain(k_sum_squares, grid_reduce(5 * (int64_t)n), s, 5 * (int64_t)n, res, rms);
   return launch_status("calc_rms");
 }
 
@@ -555,7 +548,7 @@ extern "C" int mgcfd_op_count_bad_vals(int32_t n, const double* v, int32_t* coun
   CHECK_PTR(v, n, "count_bad_vals");
   if (!count) return set_error(MGCFD_ERR_INVALID, "mgcfd_op_count_bad_vals: null output");
   if (n == 0) return MGCFD_OK;
-  launch(k_count_bad, grid_reduce(5 * (int64_t)n), kThreads, STREAM(s), false, 5 * (int64_t)n, v, count);
+  chain(k_count_bad, grid_reduce(5 * (int64_t)n), s, 5 * (int64_t)n, v, count);
   return launch_status("count_bad_vals");
 }
 

@@ -132,6 +132,7 @@ struct Scratch {
   explicit Scratch(cudaStream_t st) : s(st) {}
   ~Scratch() {
     for (void* p : ptrs) cudaFreeAsync(p, s);
+    if (!ptrs.empty()) after_free(s);
   }
   template <class T>
   int get(T** p, size_t count) {
