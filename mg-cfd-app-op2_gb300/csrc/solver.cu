@@ -2170,6 +2170,7 @@ void free_solver(mgcfd_solver* s) {
   for (auto& ev : s->pending) { cudaEventDestroy(ev.first); cudaEventDestroy(ev.second); }
   for (auto& ev : s->spare) { cudaEventDestroy(ev.first); cudaEventDestroy(ev.second); }
   for (void* p : s->allocs) cudaFreeAsync(p, s->stream);
+  if (s->stream && !s->owns_stream) after_free(s->stream);  // the caller's stream lives on
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->owns_stream) cudaStreamDestroy(s->stream);
   delete s;

@@ -64,3 +64,20 @@ def test_plans_built_on_live_streams_leave_setup_alone(form):
         for e in maps:
             ops.plan_release(e.data_ptr())
     assert after < 2 * before, (before, after)
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_solvers_closed_on_live_streams_leave_setup_alone(use_graph):
+    """Solvers closed on 32 streams of the caller's, run from their graph or
+    launch by launch: a later set-up takes what it took before (it took 5 times
+    as long; twice is the line)."""
+    mesh = mgcfd.HostMesh.generate(24, 3, 6)
+    streams = _streams()
+    before = _create_seconds()
+    for q in streams:
+        s = mgcfd.Solver(mesh, 0.5, 3.0, precision="mixed", use_graph=use_graph, stream=q.cuda_stream)
+        s.run(4)
+        assert s.synchronize() == 0
+        s.close()
+    after = _create_seconds()
+    assert after < 2 * before, (before, after)
