@@ -134,12 +134,15 @@ __device__ __forceinline__ double div_fast(double a, double b) {
   return fma(fma(-q, b, a), y, q);
 }
 
-// a / b for finite a with y = rcp_fast(b), for several quotients by one b: q = a y
-// is within 2 ulp, the remainder a - b q exact, and the last step within
-// 0.5 + 2^-52 ulp (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): the IEEE quotient
-// unless a / b lies within 2^-52 ulp of a rounding tie.  The same ranges as
-// div_fast.  3 FP64 operations.
+// a / b for finite a with y = 1 / b correctly rounded, for several quotients by
+// one b: the IEEE quotient (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  With
+// B < 2 the significand of b, b y is within B 2^-54 of 1, so a q = a y that
+// misses a / b by d ulp leaves d B 2^-54 ulp before the last rounding, while a / b
+// is no closer than 2^-53 / B ulp to a tie.  Ties lie at d = 1/2, where B^2 < 4 is
+// enough, and at d = 3/2, which q reaches only with both significands within
+// 2^-50 of 2 (checked one by one).  A y a unit off (rcp_fast's, for b just below
+// a power of two) loses that.  The same ranges as div_fast.  3 FP64 operations.
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   uint32_t ahi, alo, hi, lo;
   unpack_words(a, ahi, alo);

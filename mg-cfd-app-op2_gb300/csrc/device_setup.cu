@@ -289,7 +289,7 @@ __global__ void k_edge_geometry(int32_t ne, Seg g, const int32_t* __restrict__ e
   // (Six quotients by one distance: IEEE divisions were 60% of this kernel, 204
   // us at 774K edges; a 64^3 FP64 set-up went from 2.25 to 2.04 ms with these and
   // the shorter sort keys.)
-  const double y = rcp_fast(dist);
+  const double y = 1.0 / dist;
   for (int i = 0; i < 3; i++)
     w[3 * e + i] = __dmul_rn(div_by(__dmul_rn(div_by(d[i], dist, y), area), dist, y), 1e-7);
 }
