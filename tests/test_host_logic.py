@@ -71,6 +71,24 @@ def test_autotune_skips_failed_candidates():
     assert (best["increment"], best["block_size"]) == ("gather", 128)
 
 
+def test_autotune_tries_a_plain_fp64_solvers_own_choice(monkeypatch):
+    """Small FP64 meshes have a form that no explicit increment names; batches have
+    not, and neither has another precision."""
+    table = {("auto", 0): 1, ("atomic", 128): 20, ("atomic", 256): 25, ("gather", 128): 25, ("gather", 256): 25,
+             ("fused", 0): 15}
+    made = maker(table)
+    monkeypatch.setattr(autotune, "Solver", lambda mesh, mach, aoa, **o: made(**o))
+    monkeypatch.setattr(autotune, "Batch", lambda meshes, machs, aoas, **o: made(**o))
+    mesh = mgcfd.HostMesh.generate(4, 1, 1)
+    best, timings = autotune.tune_solver(mesh, 0.5, 2.0, cycles=1)
+    assert best == {"increment": "auto", "block_size": 0, "precision": "fp64"} and len(timings) == 5
+    best, timings = autotune.tune_solver(mesh, 0.5, 2.0, precision="mixed", cycles=1)
+    assert best["increment"] == "fused" and len(timings) == 5
+    autotune._CACHE.clear()
+    best, timings = autotune.tune_batch([mesh, mesh], [0.5] * 2, [2.0] * 2, cycles=1)
+    assert best["increment"] == "atomic" and len(timings) == 4
+
+
 def test_autotune_caches_by_size_class_and_precision():
     table = {("atomic", 128): 1, ("atomic", 256): 2, ("gather", 128): 2, ("gather", 256): 2, ("fused", 0): 2}
     first = autotune.tune(maker(table), 1000, "fp64", cycles=1)
