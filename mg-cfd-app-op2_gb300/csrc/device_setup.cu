@@ -746,7 +746,6 @@ int build_level(mgcfd_solver* s, cudaStream_t st, Temp& tmp, const Seg& g, const
 
 int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
   cudaStream_t st = s->stream;
-  const bool mixed = s->opt.precision == MGCFD_PRECISION_MIXED;
   const int nseg = (int)meshes.size();
   const int nlevels = (int)s->L.size();
   int r;

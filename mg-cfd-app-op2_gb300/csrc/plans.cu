@@ -270,11 +270,6 @@ __global__ void k_place_rest(int32_t nn, int32_t base, const int32_t* __restrict
   order[p] = (int32_t)i;
 }
 
-__global__ void k_iota(int32_t n, int32_t* __restrict__ v) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = (int32_t)i;
-}
-
 // Internal endpoints of every edge; invalid edges sort last.
 __global__ void k_edge_keys(int32_t ne, int32_t nn, const int32_t* __restrict__ e2n, const int32_t* __restrict__ pos,
                             unsigned long long* __restrict__ key, int32_t* __restrict__ val) {
