@@ -343,13 +343,18 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
 
 // A sum of binary32 terms kept exactly enough to stand for an FP64 one, on
 // the FP32 pipe: hi runs the TwoSum chain, its errors run a second TwoSum
-// chain in lo, and the errors of that collect in tail.  hi + lo + tail is within
-// n^2 2^-72 of the exact sum of n terms relative to their magnitudes, where
-// adding the terms in FP64 loses up to 2^-53 each; the value is rounded to
-// FP64 at the end.  13 FP32 operations a term against one FP64 addition, which
-// issues 64 times as slowly on GB300 (200^3 mixed V-cycle: 3.50 ms with FP64
-// additions, 2.99 with these).  A sum that leaves binary32's range, or
-// has a term that is not finite, ends as hi, infinite or NaN.
+// chain in lo, and the errors of that collect in tail.  With M the sum of n
+// terms' magnitudes, a step's error is at most 2^-24 M, so |lo| <= n 2^-24 M,
+// |tail| <= n^2/2 2^-48 M and, tail being rounded once a term, hi + lo + tail is
+// within n^3/6 2^-72 M of the exact sum: below the n 2^-53 M that adding the
+// terms in FP64 may lose for up to 1700 terms, more than a mesh node has edges.
+// The value is rounded to FP64 at the end.  13 FP32 operations a term against
+// one FP64 addition, which issues 64 times as slowly on GB300 (200^3 mixed
+// V-cycle: 3.50 ms with FP64 additions, 2.99 with these).  A sum that leaves
+// binary32's range, or has a term that is not finite, ends as hi, infinite or
+// NaN.  Fluxes cannot get there: an edge weight of 2^64 is infinite in its FP32
+// magnitude already, and above Mach 5000 or so FP32 has no digit of the pressure
+// left beside the energy, so a flux stays below 1e31.
 struct Sum32 {
   float hi, lo, tail;
 };

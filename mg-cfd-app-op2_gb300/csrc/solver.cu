@@ -497,7 +497,10 @@ __global__ void k_dw_table_b(int32_t ne, const int2* __restrict__ e2n, const int
 // round, which the L1 pipe paid for (DW at 100^3: 70% of its wavefronts).
 // V-cycle at 100^3, CSR -> sliced: DW 624 -> 584 us, pair sums 472 -> 460, mixed
 // 514 -> 509; at 200^3 3.56 -> 3.47, 2.63 -> 2.57 and 2.90 -> 2.91 ms (there
-// the FP64 node sums' tail, not the lists, holds the mixed stage).  A node's entries keep the gather order,
+// the FP64 node sums' tail, not the lists, holds the mixed stage).  Only meshes
+// whose neighbouring nodes have about as many edges get them (build_slices):
+// lattices do, tetrahedral meshes of scattered points do not.  A node's entries
+// keep the gather order,
 // its a-side edges then its b-side ones; the b side has h negated and bit 31 of
 // the id set.
 template <bool DW>
@@ -760,10 +763,11 @@ __device__ __forceinline__ void settle_halt(int halt, DevStatus* st) {
 // solvers mark the failing mesh and leave the others running.  The fused
 // stage with pair sums is latency-bound: capped at 48 registers (10 blocks
 // per SM, a few bytes spilled) it runs 2% faster; the DW stage capped at 64
-// (8 blocks, no spill) 1.5% faster than at its own 72, and slower at 56
-// (spills); the last mixed stage over sliced lists capped at 56 (9 blocks; it
-// takes 63) 2% of the V-cycle faster (200^3 2.88 -> 2.81 ms, 100^3 503 -> 495 us),
-// and slower on small levels when capped further.  Every other form keeps the
+// (8 blocks; over sliced lists 8 bytes spilled, 36 in a batch's last stage) 1.5%
+// faster than at its own 72, and slower at 56; the last mixed stage over sliced
+// lists capped at 56 (9 blocks; it takes 63, 16 bytes spilled) 2% of the V-cycle
+// faster (200^3 2.88 -> 2.81 ms, 100^3 503 -> 495 us), and slower on small levels
+// when capped further.  Every other form keeps the
 // compiler's own register choice: a minimum of 0 blocks is no constraint,
 // whereas a minimum of 1 lets it grow to 70-80 registers and lose occupancy.
 // Fused stage, STAGE (option stage_neighbour_ids): the block's neighbour ids

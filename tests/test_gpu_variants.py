@@ -152,6 +152,24 @@ def test_sum32_is_no_worse_than_fp64_adds(native, terms):
     assert err.sum() <= np.abs(seq.astype(np.longdouble) - exact).sum() * (1 + 1e-9) + float(bound.sum()) * 1e-3
 
 
+@pytest.mark.parametrize("terms", [41, 300, 1700])
+@pytest.mark.parametrize("signs", ["one", "both"])
+def test_sum32_of_many_terms(native, terms, signs):
+    """... and for nodes with many edges: n^3/6 2^-72 of the terms' magnitudes (each
+    of the three words' rounding added up), half an ulp of the value, and 2^-53 of
+    lo + tail, itself n 2^-24 of the magnitudes."""
+    rng = np.random.default_rng(terms)
+    n = 4_000
+    x = rng.random((n, terms)) if signs == "one" else rng.random((n, terms)) * 2 - 1
+    x = x.astype(np.float32)
+    out = np.empty(n)
+    assert native.sum_check(C.c_int64(n), C.c_int(terms), x.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p)) == 0
+    exact = x.astype(np.longdouble).sum(axis=1)
+    mag = np.abs(x).astype(np.longdouble).sum(axis=1)
+    bound = np.abs(exact) * 2.0 ** -53 + mag * (terms ** 3 / 6 * 2.0 ** -72 + terms * 2.0 ** -77 + terms * 2.0 ** -63)
+    assert (np.abs(out.astype(np.longdouble) - exact) <= bound).all()
+
+
 def test_sum32_beyond_binary32_and_not_finite(native):
     f = np.float32
     x = np.array([[np.inf, 1], [-np.inf, 1], [np.inf, -np.inf], [np.nan, 1], [3e38, 3e38], [-3e38, -3e38], [0.0, -0.0],
