@@ -29,6 +29,7 @@
 // kernel.
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -49,20 +50,17 @@ int bits_for(int64_t n) {  // number of bits needed to hold values 0..n
   return b;
 }
 
-// Setup scratch: a bump allocator over stream-ordered chunks, so that the many
-// temporaries of a setup cost a handful of allocation calls.  A chunk is what
-// the setup is going to need (level_scratch), 64 MiB at most unless one
-// temporary is larger: chunks of 64 MiB throughout held 128 MiB for the two
-// streams of a 21^3 mesh's setup, which needs 8 MB.  Everything is released when
-// the setup ends.
+// Setup scratch: a bump allocator over stream-ordered chunks of at least
+// `chunk` bytes, so that the many temporaries of a setup cost a handful of
+// allocation calls.  Everything is released when the setup ends.
 struct Temp {
-  static constexpr size_t kMaxChunk = 64ull << 20;
+  static constexpr size_t kChunk = 64ull << 20;
   cudaStream_t stream;
   size_t chunk;
   std::vector<void*> chunks;
   char* cur = nullptr;
   size_t left = 0;
-  Temp(cudaStream_t s, size_t need) : stream(s), chunk(need < kMaxChunk ? need : kMaxChunk) {}
+  explicit Temp(cudaStream_t s, size_t least = kChunk) : stream(s), chunk(least) {}
   ~Temp() {
     for (void* p : chunks) cudaFreeAsync(p, stream);
   }
@@ -568,14 +566,10 @@ struct SideStream {
 // nodes on.
 constexpr int32_t kSideNodes = 8192;
 
-// Bytes that build_level takes from its Temp, and those of the level's inputs
-// and multigrid tables: the arrays below and the sorts' work space (one more
-// copy of what is sorted), with 128 KiB for the rounding of each.
+// Bytes that build_level takes from its Temp: the arrays below and the sorts'
+// work space (one more copy of what is sorted), with 128 KiB for rounding.
 size_t level_scratch(int64_t n, int64_t ne, int64_t nb, bool batched) {
   return (size_t)((batched ? 97 : 69) * n + 180 * ne + 24 * nb + (128 << 10));
-}
-size_t level_inputs(int64_t n, int64_t ne, int64_t nb) {
-  return (size_t)(64 * n + 32 * ne + 32 * nb + (16 << 10));
 }
 
 // One level's tables and state, from its inputs, on stream st with scratch
@@ -775,13 +769,7 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
   std::vector<mgcfd_freestream> ffs((size_t)nseg);
   for (int m = 0; m < nseg; m++) ffs[(size_t)m] = meshes[(size_t)m].ff;
   auto total = [&](int l, int which) { return meta[per * (size_t)l + (size_t)which * (nseg + 1) + (size_t)nseg]; };
-  const bool two_streams = nlevels > 1 && total(0, 0) >= kSideNodes;  // the coarse levels beside level 0, below
-  size_t need = 4 * meta.size() + sizeof(mgcfd_freestream) * (size_t)nseg, side_need = 0;
-  for (int l = 0; l < nlevels; l++) {
-    need += level_inputs(total(l, 0), total(l, 1), total(l, 2));
-    (two_streams && l > 0 ? side_need : need) += level_scratch(total(l, 0), total(l, 1), total(l, 2), nseg > 1);
-  }
-  Temp tmp(st, need);
+  Temp tmp(st);
   int32_t* dmeta;
   mgcfd_freestream* dff;
   unsigned* fin;  // fin[0]: out-of-range map entries; fin[1 + l]: folded boundary rows of level l, then slice rows
@@ -836,8 +824,15 @@ int device_prepare(mgcfd_solver* s, const std::vector<MeshInput>& meshes) {
   // multigrid tables.  (64^3 FP64: 2.03 -> 1.77 ms, 48^3 1.58 -> 1.34.)  On
   // smaller meshes the host's launches take the time, and one stream is enough.
   SideStream side;
-  if (two_streams && (r = side.open(st))) return r;
-  Temp side_tmp(side.stream ? side.stream : st, side_need);
+  if (nlevels > 1 && total(0, 0) >= kSideNodes && (r = side.open(st))) return r;
+  // The second arena in a chunk of what the coarse levels need, so that a set-up
+  // on two streams holds little more than one on one did (a second chunk of 64
+  // MiB: 133 MB beyond the solver's own for 21^3).  The first keeps its 64 MiB:
+  // chunks by need there left the pool to grow for each solver that a program
+  // keeps (10 solvers of 48^3 nodes: 9.1 -> 10.4 ms to make one).
+  size_t side_need = 0;
+  for (int l = 1; l < nlevels; l++) side_need += level_scratch(total(l, 0), total(l, 1), total(l, 2), nseg > 1);
+  Temp side_tmp(side.stream ? side.stream : st, std::min(side_need, Temp::kChunk));
   for (int l = 0; l < nlevels; l++) {
     const bool beside = side.stream && l > 0;
     if ((r = build_level(s, beside ? side.stream : st, beside ? side_tmp : tmp, seg(l), in[(size_t)l], l, total(l, 0),

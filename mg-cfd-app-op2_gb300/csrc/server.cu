@@ -164,7 +164,7 @@ int64_t estimate_bytes(const std::vector<mgcfd_level_view>& lv, int precision, i
     // (The fused stage's sliced edge lists, up to 2.5 entries of 20 or 36 bytes
     // per edge, are built when the set-up scratch below, 120 bytes per edge, has
     // been freed: the peak stays the set-up's.  That scratch comes in chunks of
-    // what the levels need, on one stream or two.)
+    // at least 64 MiB; a set-up on two streams adds what its coarse levels need.)
     if (dw) {  // rec2, w4dw; fused: rec2b, off2, ent2
       node += 64 + (fused ? 68 : 0);
       edge += 32 + (fused ? 16 : 0);

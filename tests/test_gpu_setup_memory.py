@@ -34,11 +34,12 @@ def pool():
 # One stream, two streams (from 8192 level-0 nodes), and one with the lists of the fused stage.
 @pytest.mark.parametrize("n,nl", [(8, 3), (21, 3), (40, 4)])
 @pytest.mark.parametrize("precision", ["fp64", "mixed", "dw"])
-def test_scratch_is_what_the_levels_need(pool, n, nl, precision):
-    """Beyond what the solver keeps, a set-up holds at most 1100 bytes per level-0
-    node of a lattice (three edges a node: 64 + 3 * 32 bytes of inputs and 69 +
-    3 * 180 of work space, a seventh more for the coarse levels, and up to 60 bytes
-    for each of the surface's entries) and 1 MiB of rounding."""
+def test_scratch_of_two_streams_is_little_more_than_one_chunk(pool, n, nl, precision):
+    """Beyond what the solver keeps, a set-up holds one chunk of 64 MiB and what its
+    coarse levels need: on a lattice (three edges a node) at most 69 + 3 * 180 and
+    up to 60 bytes for each of the surface's entries, so 900 bytes for each of the
+    n^3 / 7 coarse nodes (a little more of odd extents: n^3 / 5), and 1 MiB of
+    rounding."""
     get, reset_high = pool
     mesh = mgcfd.HostMesh.generate(n, nl, 5)
     torch.cuda.synchronize()
@@ -47,4 +48,4 @@ def test_scratch_is_what_the_levels_need(pool, n, nl, precision):
     s = mgcfd.Solver(mesh, 0.5, 3.0, precision=precision)
     peak, kept = get(USED_HIGH) - before, s.stats().device_bytes
     s.close()
-    assert peak - kept < 1100 * n ** 3 + (1 << 20), (peak, kept)
+    assert peak - kept < (64 << 20) + 900 * n ** 3 // 5 + (1 << 20), (peak, kept)
